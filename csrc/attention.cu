@@ -4,8 +4,8 @@
 // `parallel_blocks` split-KV and `flash_attn_combine_results` (fattn-common.cuh:721-772).  The reference
 // cache is a contiguous ring per stream; here K/V live in fixed-size pages
 // [n_pages][Hkv][page_size][D] addressed through a block table, so sequences grow without copies and
-// TP ranks own disjoint KV heads.  One CTA = (split, kv head [x q-head group], query); the G <= 4 query
-// heads that share a KV head are processed together so each K/V byte is read once per group.
+// TP ranks own disjoint KV heads.  One CTA = (split, kv head [x q-head group], query); the query heads that
+// share a KV head are processed together so each K/V byte is read once per group.
 #include "kernels.cuh"
 #include <cooperative_groups.h>
 
@@ -21,151 +21,380 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int D, int G>
-__global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
-    constexpr int DL = D / 8;  // dims per lane (8 lanes share one token)
-    static_assert(DL % 8 == 0, "head dim must be a multiple of 64");
-    const int split = blockIdx.x;
-    const int groups_per_kv = (p.Hq / p.Hkv) / G;
-    const int kvh = blockIdx.y / groups_per_kv;
-    const int hq0 = kvh * (p.Hq / p.Hkv) + (blockIdx.y % groups_per_kv) * G;
-    const int qi = blockIdx.z;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grp = lane >> 3, sub = lane & 7;
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem)));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem)));
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
+    __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ uint32_t movmatrix(uint32_t a) {      // 8 x 8 halves, two of a row per lane, transposed
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+// two fp32 values as fp16 pairs: value and remainder (22 bits together)
+__device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = pack_h2(a - f.x, b - f.y);
+}
 
+// ---- split-KV attention on the tensor cores ------------------------------------------------------------------------------
+// Bound by the bytes of K and V: one CTA = (split of the keys, KV head, query); the query heads that share the KV head are the 8 columns of
+// mma.sync m16n8k16 (a query has too few heads for a tcgen05 tile), 16 keys (then 16 dims of V, transposed by ldmatrix) its rows, so every
+// K / V byte is read once.  (Heads as the 16 rows: half of the tile is padding, twice the MMAs.)  Each of the 4 warps streams its own tiles of 16 keys through a private ring of
+// 3 stages (cp.async, 8 KB a stage at D = 128; 2 CTAs an SM: 128 KB in flight) and keeps its own running maximum; page ids are fetched one
+// tile ahead; the warps are merged through shared memory, the splits by the last CTA of the (query, head) to finish.
+// Scores and sums are fp32; the softmax weights (and with ROPE the rotated fp32 queries) enter the tensor cores as two fp16 parts, value and
+// remainder, in units of 2^-10 so that the remainder of small weights is not lost to subnormals.
+// 32,000 keys of 8 KV heads of 4 query heads, D = 128 (131 MB): 28.5 us (4.6 TB/s; 108 us with fp32 FMA per key in 128 CTAs); 32 queries
+// of up to 2,000 keys (135 MB): 34 us (117 us).
+//   ROPE: takes the fp32 row of the QKV mat-vec, rotates q in registers, writes the new token's K and V and uses them from shared memory.
+constexpr int ATTN_KEYS_MIN = 128;      // keys a split is worth: 2 tiles per warp, all requested before the dependency wait (700 keys in a
+                                        // decode step: as fast as the cluster form; with 256 keys 1.7 us slower)
+struct AttnRange { int eff, begin, end; };
+__device__ __forceinline__ AttnRange attn_range(int len, int n_splits, int split) {
+    AttnRange r;
+    const int want = min(n_splits, max(1, (len + ATTN_KEYS_MIN - 1) / ATTN_KEYS_MIN));
+    const int per = max(16, ((len + want - 1) / want + 15) & ~15);      // whole tiles
+    r.eff = max(1, (len + per - 1) / per);
+    r.begin = split * per;
+    r.end = min(len, r.begin + per);
+    return r;
+}
+struct AttnRope {
+    const float* qkv;          // [nq][(Hq + 2 Hkv) * D], not rotated
+    const float* inv_freq;     // [D / 2], or
+    const float2* cs;          // [nq][D / 2] (cos, sin)
+    __half* kc_w;
+    __half* vc_w;
+    int neox;
+    float q_scale;
+};
+
+// One warp joins the partials of `eff` splits of one (query, head): a lane takes D / 32 dims, its loads of 8 splits in flight at a time.
+// (Maxima are in units of log 2.  One thread per dim, splits one after the other: 45 us instead of 28.5 for 32,000 keys in 37 splits.)
+template <int D>
+__device__ __forceinline__ void attn_join(const AttnParams& p, size_t head, int eff, int lane) {
+    constexpr int E = D / 32;
+    const size_t pi0 = head * p.n_splits;
+    const float* ml = p.part_ml + pi0 * 2;
+    float mn = -INFINITY, ls = 0.f, acc[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) acc[i] = 0.f;
+    for (int s = lane; s < eff; s += 32) mn = fmaxf(mn, __ldcg(ml + 2 * s));
+    mn = warp_max(mn);
+    for (int s0 = 0; s0 < eff; s0 += 32) {
+        const float2 v = s0 + lane < eff ? make_float2(__ldcg(ml + 2 * (s0 + lane)), __ldcg(ml + 2 * (s0 + lane) + 1)) : make_float2(-INFINITY, 0.f);
+        const float a = v.x == -INFINITY ? 0.f : exp2f(v.x - mn);
+        ls += v.y * a;
+        const int n = min(32, eff - s0);
+        for (int s = 0; s < n; s += 8) {
+            float x[8][E];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float* src = p.part_o + (pi0 + s0 + min(s + u, n - 1)) * D + lane;
+#pragma unroll
+                for (int i = 0; i < E; ++i) x[u][i] = __ldcg(src + 32 * i);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float w = __shfl_sync(0xffffffffu, a, min(s + u, 31));
+#pragma unroll
+                for (int i = 0; i < E; ++i) if (s + u < n) acc[i] = fmaf(x[u][i], w, acc[i]);
+            }
+        }
+    }
+    ls = warp_sum(ls);
+    const float inv = ls > 0.f ? 1.f / ls : 0.f;
+#pragma unroll
+    for (int i = 0; i < E; ++i) p.out[head * D + lane + 32 * i] = __float2half_rn(acc[i] * inv);
+}
+
+template <int D> constexpr int attn_split_smem() { return 4 * 3 * 2 * 16 * D * 2; }      // warps x stages x (K, V) x keys x D (the merge needs 4 x 16 x (D + 2) floats of it)
+
+template <int D, int NH, bool ROPE>      // NH: groups of 8 query heads in use
+__global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, const AttnRope ra) {
+    constexpr int STAGES = 3, KS = D / 16, CPR = D / 8, TILE = 16 * D * 2;      // k steps, 16-byte chunks per row, bytes of one K or V tile
+    constexpr float LOG2E = 1.4426950408889634f, UP = 10.f;
+    extern __shared__ __align__(128) uint8_t as_smem[];
+    const int gqa = p.Hq / p.Hkv, R = 8 * NH, groups = (gqa + R - 1) / R;
+    const int kvh = blockIdx.y / groups, h0 = (blockIdx.y % groups) * R, G = min(R, gqa - h0), hq0 = kvh * gqa + h0;
+    const int split = blockIdx.x, qi = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     trace_event(p.trace, TR_ATTN | TR_BEGIN);
-    pdl_wait();
-    trace_event(p.trace, TR_ATTN | TR_WAITED);
+    // ROPE: length, pages and the cached rows were written at least two launches back (the immediate predecessor is the QKV mat-vec), so
+    // the first tiles are requested before the dependency wait.  Otherwise the predecessor wrote the newest K / V row.
+    if (!ROPE) pdl_wait();
     const int len = p.kv_len[qi];
-    // effective split count grows with the context (one split per 64 keys): a short context is handled by a single CTA
-    // that writes the final result itself; the launch shape (n_splits) stays fixed so the step can live in a CUDA graph
-    const int eff = min(p.n_splits, max(1, (len + 63) / 64));
-    if (split >= eff) return;
-    const int per = (len + eff - 1) / eff;
-    const int begin = split * per, end = min(len, begin + per);
+    const AttnRange rg = attn_range(len, p.n_splits, split);
+    if (split >= rg.eff) return;
+    const int n_old = len - 1;
+    const int n_tiles = (rg.end - rg.begin + 15) >> 4, n_mine = n_tiles > warp ? (n_tiles - warp + 3) >> 2 : 0;
     const int* bt = p.block_table + (size_t)(p.bt_row ? p.bt_row[qi] : qi) * p.max_pages;
-
-    float q[G][DL];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const __half* qp = p.q + ((size_t)qi * p.Hq + hq0 + g) * D + sub * DL;
-#pragma unroll
-        for (int i = 0; i < DL; i += 8) {
-            const uint4 v = *reinterpret_cast<const uint4*>(qp + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = h2_to_f2(w[j]);
-                q[g][i + 2 * j] = f.x;
-                q[g][i + 2 * j + 1] = f.y;
-            }
-        }
-    }
-    float m[G], l[G], o[G][DL];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        m[g] = -INFINITY;
-        l[g] = 0.f;
-#pragma unroll
-        for (int i = 0; i < DL; ++i) o[g][i] = 0.f;
-    }
-
-    // warp-uniform loop bound: all 32 lanes take part in every shuffle; groups past `end` re-read the last valid
-    // token and discard the result.  The raw K/V rows of the *next* iteration are requested before the current one is
-    // reduced (the page lookup -> K/V load chain is pure latency otherwise).
-    constexpr int NV = DL / 8;   // 16-byte loads per lane and tensor
-    uint4 kr[NV], vr[NV], kn[NV], vn[NV];
-    auto fetch = [&](int tok0, uint4 (&kd)[NV], uint4 (&vd)[NV]) {
-        const int tok = min(tok0 + grp, end - 1);
-        const int page = bt[tok / p.page_size], off = tok % p.page_size;
-        const size_t base = (((size_t)page * p.Hkv + kvh) * p.page_size + off) * D + sub * DL;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            kd[i] = ldg_nc_v4(p.kc + base + i * 8);
-            vd[i] = ldg_nc_v4(p.vc + base + i * 8);
-        }
+    uint8_t* ring = as_smem + warp * (STAGES * 2 * TILE);
+    auto rows_of = [&](int j) {              // lane r < 16: element offset of row r of this warp's tile j (-1: not a cached key)
+        const int tok = rg.begin + ((j * 4 + warp) << 4) + (lane & 15);
+        if (j >= n_mine || tok >= (ROPE ? min(rg.end, n_old) : rg.end)) return (long long)-1;
+        const int pg = tok / p.page_size;
+        return (((long long)bt[pg] * p.Hkv + kvh) * p.page_size + (tok - pg * p.page_size)) * D;
     };
-    const int t_first = begin + warp * 4;
-    if (t_first < end) fetch(t_first, kr, vr);
-    for (int tok0 = t_first; tok0 < end; tok0 += 16) {
-        const bool valid = tok0 + grp < end;
-        const bool more = tok0 + 16 < end;
-        if (more) fetch(tok0 + 16, kn, vn);
-        float kf[DL], vf[DL];
+    auto issue = [&](int j, long long where) {
+        if (j < n_mine) {
+            uint8_t* st = ring + (j % STAGES) * (2 * TILE);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const uint32_t kw[4] = {kr[i].x, kr[i].y, kr[i].z, kr[i].w}, vw[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 a = h2_to_f2(kw[j]), b = h2_to_f2(vw[j]);
-                kf[i * 8 + 2 * j] = a.x; kf[i * 8 + 2 * j + 1] = a.y;
-                vf[i * 8 + 2 * j] = b.x; vf[i * 8 + 2 * j + 1] = b.y;
+            for (int i = 0; i < CPR / 2; ++i) {
+                const int e = i * 32 + lane, r = e / CPR, c = e % CPR;
+                const long long o = __shfl_sync(0xffffffffu, where, r);
+                const int at = r * (D * 2) + ((c ^ (r & 7)) << 4);
+                cp_async16(st + at, p.kc + (o < 0 ? 0 : o + c * 8), o >= 0);
+                cp_async16(st + TILE + at, p.vc + (o < 0 ? 0 : o + c * 8), o >= 0);
             }
         }
+        cp_async_commit();
+    };
+    issue(0, rows_of(0));
+    issue(1, rows_of(1));
+    long long where = rows_of(2);
+    if (ROPE) {
+        pdl_wait();
+        if (p.pdl_early) pdl_launch_dependents();
+    }
+    trace_event(p.trace, TR_ATTN | TR_WAITED);
+
+    // queries as B fragments: head g, dims ks * 16 + 2t, + 1 and + 8, + 9
+    uint32_t qh[KS][NH][2], ql[ROPE ? KS : 1][NH][2];
+    const float2* cs_tab = ROPE && ra.cs ? ra.cs + (size_t)qi * (D / 2) : nullptr;
+    auto angle = [&](int i) {               // (cos, sin) of pair i
+        if (cs_tab) return cs_tab[i];
+        float2 v;
+        sincosf((float)n_old * ra.inv_freq[i], &v.y, &v.x);
+        return v;
+    };
+    const float* row = ROPE ? ra.qkv + (size_t)qi * (p.Hq + 2 * p.Hkv) * D : nullptr;
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float s = 0.f;
+    for (int nh = 0; nh < NH; ++nh) {
+        const int r = nh * 8 + g;
+        if constexpr (ROPE) {
+            const float* src = row + (size_t)(hq0 + min(r, G - 1)) * D;
+            float2 x[KS][2];
 #pragma unroll
-            for (int i = 0; i < DL; ++i) s = fmaf(q[g][i], kf[i], s);
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            if (!valid) continue;
-            const float mn = fmaxf(m[g], s);
-            const float alpha = __expf(m[g] - mn), pr = __expf(s - mn);
-            m[g] = mn;
-            l[g] = l[g] * alpha + pr;
+            for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-            for (int i = 0; i < DL; ++i) o[g][i] = fmaf(pr, vf[i], o[g][i] * alpha);
-        }
-        if (more) {
+                for (int e = 0; e < 2; ++e) x[ks][e] = *reinterpret_cast<const float2*>(src + ks * 16 + e * 8 + 2 * t);
+            if (ra.neox) {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) { kr[i] = kn[i]; vr[i] = vn[i]; }
+                for (int ks = 0; ks < KS / 2; ++ks)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 a = angle(ks * 16 + e * 8 + 2 * t), b = angle(ks * 16 + e * 8 + 2 * t + 1), u = x[ks][e], v = x[ks + KS / 2][e];
+                        x[ks][e] = make_float2(u.x * a.x - v.x * a.y, u.y * b.x - v.y * b.y);
+                        x[ks + KS / 2][e] = make_float2(v.x * a.x + u.x * a.y, v.y * b.x + u.y * b.y);
+                    }
+            } else {
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 a = angle(ks * 8 + e * 4 + t), u = x[ks][e];
+                        x[ks][e] = make_float2(u.x * a.x - u.y * a.y, u.x * a.y + u.y * a.x);
+                    }
+            }
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float sc = r < G ? ra.q_scale : 0.f;
+                    split_h2(x[ks][e].x * sc, x[ks][e].y * sc, qh[ks][nh][e], ql[ks][nh][e]);
+                }
+        } else {
+            const __half* src = p.q + ((size_t)qi * p.Hq + hq0 + min(r, G - 1)) * D;
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const uint32_t v = *reinterpret_cast<const uint32_t*>(src + ks * 16 + e * 8 + 2 * t);
+                    qh[ks][nh][e] = r < G ? v : 0u;
+                }
         }
     }
+    float o[D / 16][NH][4];                  // dims g and g + 8 of a group of 16, heads 2t and 2t + 1
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i)
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh) { o[i][nh][0] = o[i][nh][1] = o[i][nh][2] = o[i][nh][3] = 0.f; }
+    float m[NH][2], l[NH][2];
+#pragma unroll
+    for (int nh = 0; nh < NH; ++nh) { m[nh][0] = m[nh][1] = -INFINITY; l[nh][0] = l[nh][1] = 0.f; }
+    const int mat = lane >> 3, r8 = lane & 7;
+    for (int j = 0; j < n_mine; ++j) {
+        const long long next = rows_of(j + 3);
+        issue(j + 2, where);                 // (its stage was read in iteration j - 1)
+        where = next;
+        cp_async_wait_group<2>();
+        __syncwarp();
+        uint8_t* sK = ring + (j % STAGES) * (2 * TILE);
+        uint8_t* sV = sK + TILE;
+        const int tok0 = rg.begin + ((j * 4 + warp) << 4);
+        if (ROPE && n_old >= tok0 && n_old < min(tok0 + 16, rg.end)) {      // the new token: rotate K, round K and V to the cache's type, into the tile and into the page
+            constexpr int E = D / 32;
+            const float* ks_ = row + (size_t)(p.Hq + kvh) * D + lane * E;
+            const float* vs_ = ks_ + (size_t)p.Hkv * D;
+            float kx[E], vx[E];
+#pragma unroll
+            for (int i = 0; i < E; ++i) { kx[i] = ks_[i]; vx[i] = vs_[i]; }
+            if (ra.neox) {
+#pragma unroll
+                for (int i = 0; i < E; ++i) {
+                    const float other = __shfl_xor_sync(0xffffffffu, kx[i], 16);
+                    const float2 a = angle((lane & 15) * E + i);
+                    kx[i] = lane < 16 ? kx[i] * a.x - other * a.y : kx[i] * a.x + other * a.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < E; i += 2) {
+                    const float2 a = angle((lane * E + i) >> 1);
+                    const float u = kx[i], v = kx[i + 1];
+                    kx[i] = u * a.x - v * a.y;
+                    kx[i + 1] = u * a.y + v * a.x;
+                }
+            }
+            const int r = n_old - tok0, pg = n_old / p.page_size;
+            const int at = r * (D * 2) + ((((lane * E) >> 3) ^ (r & 7)) << 4) + ((lane * E) & 7) * 2;
+            const size_t gl = (((size_t)bt[pg] * p.Hkv + kvh) * p.page_size + (n_old - pg * p.page_size)) * D + lane * E;
+#pragma unroll
+            for (int i = 0; i < E; i += 2) {
+                const uint32_t kk = pack_h2(kx[i], kx[i + 1]), vv = pack_h2(vx[i], vx[i + 1]);
+                *reinterpret_cast<uint32_t*>(sK + at + i * 2) = kk;
+                *reinterpret_cast<uint32_t*>(sV + at + i * 2) = vv;
+                if (h0 == 0) {
+                    *reinterpret_cast<uint32_t*>(ra.kc_w + gl + i) = kk;
+                    *reinterpret_cast<uint32_t*>(ra.vc_w + gl + i) = vv;
+                }
+            }
+            __syncwarp();
+        }
+        constexpr int CHAINS = ROPE ? 4 : 2;      // independent accumulators: an MMA waits for the one before it in its chain
+        float s[NH][CHAINS][4];
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+            for (int c = 0; c < CHAINS; ++c) { s[nh][c][0] = s[nh][c][1] = s[nh][c][2] = s[nh][c][3] = 0.f; }
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+            uint32_t ka[4];
+            const int kr = (mat & 1) * 8 + r8, c = ks * 2 + (mat >> 1);
+            ldmatrix_x4(ka, sK + kr * (D * 2) + ((c ^ (kr & 7)) << 4));
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh) {
+                mma_16816(s[nh][ks & 1], ka, qh[ks][nh][0], qh[ks][nh][1]);
+                if constexpr (ROPE) mma_16816(s[nh][2 + (ks & 1)], ka, ql[ks][nh][0], ql[ks][nh][1]);
+            }
+        }
+        uint32_t ph[NH][2], pl[NH][2];       // weights as B fragments: head g, keys 2t, 2t + 1 and + 8, + 9
+        float alpha[NH][2];
+        bool grew = false;
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh) {
+            float v[4], pr[4];               // keys g (0, 1) and g + 8 (2, 3), heads 2t (even) and 2t + 1
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float x = s[nh][0][e] + s[nh][1][e];
+                if constexpr (ROPE) x += s[nh][2][e] + s[nh][3][e];
+                v[e] = tok0 + g + (e >> 1) * 8 < rg.end ? x * LOG2E : -INFINITY;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float mx = fmaxf(v[h], v[2 + h]);
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                const float mn = fmaxf(m[nh][h], mx), off = mn == -INFINITY ? 0.f : mn - UP;
+                alpha[nh][h] = m[nh][h] == -INFINITY ? 0.f : exp2f(m[nh][h] - mn);
+                grew = grew || alpha[nh][h] != 1.f;
+                m[nh][h] = mn;
+                pr[h] = exp2f(v[h] - off);
+                pr[2 + h] = exp2f(v[2 + h] - off);
+                l[nh][h] = l[nh][h] * alpha[nh][h] + (pr[h] + pr[2 + h]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t hi, lo;
+                split_h2(pr[2 * e], pr[2 * e + 1], hi, lo);
+                ph[nh][e] = movmatrix(hi);
+                pl[nh][e] = movmatrix(lo);
+            }
+        }
+        if (__any_sync(0xffffffffu, grew)) {
+#pragma unroll
+            for (int i = 0; i < D / 16; ++i)
+#pragma unroll
+                for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[i][nh][e] *= alpha[nh][e & 1];
+        }
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i) {
+            uint32_t va[4];
+            const int vr = (mat >> 1) * 8 + r8, c = i * 2 + (mat & 1);
+            ldmatrix_x4_trans(va, sV + vr * (D * 2) + ((c ^ (vr & 7)) << 4));
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh) {
+                mma_16816(o[i][nh], va, ph[nh][0], ph[nh][1]);
+                mma_16816(o[i][nh], va, pl[nh][0], pl[nh][1]);
+            }
+        }
+        __syncwarp();
+    }
+    cp_async_wait_all();
     trace_event(p.trace, TR_ATTN | TR_MAIN_DONE);
     pdl_launch_dependents();
-    // merge the 4 lane groups of the warp, then the 4 warps of the CTA
-    __shared__ float sm_m[4][G], sm_l[4][G];
-    __shared__ float sm_o[4][G][D];
+    __syncthreads();                         // every ring has been read: its memory takes the warps' results
+    float* sm_o = reinterpret_cast<float*>(as_smem);       // [4][R][D]
+    float* sm_ml = sm_o + 4 * R * D;                       // [4][R][2]
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
+    for (int nh = 0; nh < NH; ++nh)
 #pragma unroll
-        for (int off = 8; off <= 16; off <<= 1) {
-            const float m2 = __shfl_xor_sync(0xffffffffu, m[g], off);
-            const float l2 = __shfl_xor_sync(0xffffffffu, l[g], off);
-            const float mn = fmaxf(m[g], m2);
-            const float a1 = (m[g] == -INFINITY) ? 0.f : __expf(m[g] - mn);
-            const float a2 = (m2 == -INFINITY) ? 0.f : __expf(m2 - mn);
+        for (int h = 0; h < 2; ++h) {
+            float ls = l[nh][h];
+            ls += __shfl_xor_sync(0xffffffffu, ls, 4);
+            ls += __shfl_xor_sync(0xffffffffu, ls, 8);
+            ls += __shfl_xor_sync(0xffffffffu, ls, 16);
+            const int r = nh * 8 + 2 * t + h;
+            if (r < G) {
 #pragma unroll
-            for (int i = 0; i < DL; ++i) {
-                const float o2 = __shfl_xor_sync(0xffffffffu, o[g][i], off);
-                o[g][i] = o[g][i] * a1 + o2 * a2;
+                for (int i = 0; i < D / 16; ++i) {
+                    float* dst = sm_o + ((size_t)warp * R + r) * D + i * 16 + g;
+                    dst[0] = o[i][nh][h];
+                    dst[8] = o[i][nh][2 + h];
+                }
+                if (g == 0) { sm_ml[(warp * R + r) * 2] = m[nh][h]; sm_ml[(warp * R + r) * 2 + 1] = ls; }
             }
-            l[g] = l[g] * a1 + l2 * a2;
-            m[g] = mn;
         }
-        if (grp == 0) {
-#pragma unroll
-            for (int i = 0; i < DL; ++i) sm_o[warp][g][sub * DL + i] = o[g][i];
-            if (sub == 0) { sm_m[warp][g] = m[g]; sm_l[warp][g] = l[g]; }
-        }
-    }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
-        const int g = idx / D, d = idx % D;
-        float mn = -INFINITY;
+    for (int idx = threadIdx.x; idx < G * D; idx += 128) {
+        const int r = idx / D, d = idx % D, hq = hq0 + r;
+        float mn = -INFINITY, acc = 0.f, ls = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) mn = fmaxf(mn, sm_m[w][g]);
-        float acc = 0.f, ls = 0.f;
+        for (int w = 0; w < 4; ++w) mn = fmaxf(mn, sm_ml[(w * R + r) * 2]);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const float a = (sm_m[w][g] == -INFINITY) ? 0.f : __expf(sm_m[w][g] - mn);
-            acc += sm_o[w][g][d] * a;
-            ls += sm_l[w][g] * a;
+            const float mw = sm_ml[(w * R + r) * 2], a = mw == -INFINITY ? 0.f : exp2f(mw - mn);
+            acc += sm_o[((size_t)w * R + r) * D + d] * a;
+            ls += sm_ml[(w * R + r) * 2 + 1] * a;
         }
-        const int hq = hq0 + g;
-        if (eff == 1) {
+        if (rg.eff == 1) {
             p.out[((size_t)qi * p.Hq + hq) * D + d] = __float2half_rn(ls > 0.f ? acc / ls : 0.f);
         } else {
             const size_t pi = ((size_t)qi * p.Hq + hq) * p.n_splits + split;
@@ -174,38 +403,26 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
         }
     }
     trace_event(p.trace, TR_ATTN | TR_END);       // (CTA 0 is rarely the combining CTA: its END marks the partial write)
-    if (eff == 1 || p.counters == nullptr) return;
-    // fused LSE combine: the last split CTA of this (query, kv-head group) to finish merges all partials - no second launch
+    if (rg.eff == 1 || p.counters == nullptr) return;
+    // the last split CTA of this (query, head group) to finish merges all partials - no second launch
     __shared__ int is_last;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
         int* ctr = p.counters + (size_t)qi * gridDim.y + blockIdx.y;
         const int prev = atomicAdd(ctr, 1);
-        is_last = (prev == eff - 1);
+        is_last = (prev == rg.eff - 1);
         if (is_last) *ctr = 0;   // ready for the next launch
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
-        const int g = idx / D, d = idx % D;
-        const size_t pi0 = ((size_t)qi * p.Hq + hq0 + g) * p.n_splits;
-        float mn = -INFINITY;
-        for (int sp = 0; sp < eff; ++sp) mn = fmaxf(mn, __ldcg(p.part_ml + (pi0 + sp) * 2));
-        float acc = 0.f, ls = 0.f;
-        for (int sp = 0; sp < eff; ++sp) {
-            const float ms = __ldcg(p.part_ml + (pi0 + sp) * 2);
-            const float a = (ms == -INFINITY) ? 0.f : __expf(ms - mn);
-            acc += __ldcg(p.part_o + (pi0 + sp) * D + d) * a;
-            ls += __ldcg(p.part_ml + (pi0 + sp) * 2 + 1) * a;
-        }
-        p.out[((size_t)qi * p.Hq + hq0 + g) * D + d] = __float2half_rn(ls > 0.f ? acc / ls : 0.f);
-    }
+    for (int r = warp; r < G; r += 4) attn_join<D>(p, (size_t)qi * p.Hq + hq0 + r, rg.eff, lane);
 }
 
 // ---------------------------------------------------------------------------------------------
-// Decode step in ONE launch: RoPE on Q and on the new token's K, paged write of that token's K/V, split-KV attention over the
+// Decode step in ONE launch for callers without a workspace (attn_split_kernel is faster from 64 keys on: 3.4 against 7.5 us there, 6.6 against
+// 8.3 at 512, 7.6 against 13 at 2,048): RoPE on Q and on the new token's K, paged write of that token's K/V, split-KV attention over the
 // cache, and the split combine through distributed shared memory.
 //
 //   * The splits of one (query, KV-head group) form a thread-block CLUSTER (grid.x = cluster size = n_splits <= 16): partial
@@ -489,6 +706,12 @@ __global__ void __launch_bounds__(128) attn_decode_rope_kernel(const AttnParams 
     trace_event(p.trace, TR_ATTN | TR_END);
 }
 
+static int attn_pdl_early() {
+    static int early = -1;
+    if (early < 0) { const char* e = getenv("DLP_PDL_EARLY"); early = (e && e[0] == '0') ? 0 : 1; }
+    return early;
+}
+
 template <int D, int G>
 static int launch_attn_rope_g(const AttnParams& p, const float* qkv, const float* inv_freq, const float2* rope_cs, __half* kc_w,
                               __half* vc_w, int neox, float q_scale, cudaStream_t s) {
@@ -527,15 +750,13 @@ int attn_decode_rope(const AttnParams& p_in, const float* qkv, const float* inv_
                      __half* vc_w, int D, int neox, float q_scale, cudaStream_t s) {
     AttnParams p = p_in;
     p.trace = trace_buffer();
-    static int early = -1, kps = 0;
-    if (early < 0) {
-        const char* e = getenv("DLP_PDL_EARLY");
-        early = (e && e[0] == '0') ? 0 : 1;
+    static int kps = 0;
+    if (kps == 0) {
         const char* k = getenv("DLP_ATTN_KEYS_PER_SPLIT");
         kps = k ? atoi(k) : 32;
         if (kps < 16) kps = 16;
     }
-    p.pdl_early = early;
+    p.pdl_early = attn_pdl_early();
     p.keys_per_split = kps;
     DLP_REQUIRE(inv_freq != nullptr || rope_cs != nullptr, "attn_decode_rope: need inv_freq or a (cos, sin) table");
     DLP_REQUIRE(p.nq > 0 && p.Hq % p.Hkv == 0, "attn_decode_rope: bad head configuration Hq=%d Hkv=%d", p.Hq, p.Hkv);
@@ -548,37 +769,42 @@ int attn_decode_rope(const AttnParams& p_in, const float* qkv, const float* inv_
 template <int D>
 __global__ void attn_combine_kernel(const AttnParams p) {
     const int hq = blockIdx.x, qi = blockIdx.y;
-    const size_t pi0 = ((size_t)qi * p.Hq + hq) * p.n_splits;
     pdl_wait();
     pdl_launch_dependents();
-    const int len = p.kv_len[qi];
-    const int eff = min(p.n_splits, max(1, (len + 63) / 64));
+    const int eff = attn_range(p.kv_len[qi], p.n_splits, 0).eff;
     if (eff == 1) return;   // the single split already wrote the final output
-    float mn = -INFINITY;
-    for (int s = 0; s < eff; ++s) mn = fmaxf(mn, p.part_ml[(pi0 + s) * 2]);
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float acc = 0.f, ls = 0.f;
-        for (int s = 0; s < eff; ++s) {
-            const float ms = p.part_ml[(pi0 + s) * 2];
-            const float a = (ms == -INFINITY) ? 0.f : __expf(ms - mn);
-            acc += p.part_o[(pi0 + s) * D + d] * a;
-            ls += p.part_ml[(pi0 + s) * 2 + 1] * a;
-        }
-        p.out[((size_t)qi * p.Hq + hq) * D + d] = __float2half_rn(ls > 0.f ? acc / ls : 0.f);
-    }
+    attn_join<D>(p, (size_t)qi * p.Hq + hq, eff, threadIdx.x);
 }
 
-template <int D>
-static int launch_attn(const AttnParams& p, cudaStream_t s) {
-    const int gqa = p.Hq / p.Hkv;
-    const int G = gqa % 4 == 0 ? 4 : (gqa % 2 == 0 ? 2 : 1);
-    dim3 grid(p.n_splits, p.Hkv * (gqa / G), p.nq);
-    if (G == 4) DLP_CHECK_CUDA(launch_pdl(attn_decode_kernel<D, 4>, grid, dim3(128), 0, s, p));
-    else if (G == 2) DLP_CHECK_CUDA(launch_pdl(attn_decode_kernel<D, 2>, grid, dim3(128), 0, s, p));
-    else DLP_CHECK_CUDA(launch_pdl(attn_decode_kernel<D, 1>, grid, dim3(128), 0, s, p));
+template <int D, int NH, bool ROPE>
+static int launch_attn_split(const AttnParams& p, const AttnRope& ra, cudaStream_t s) {
+    auto kern = attn_split_kernel<D, NH, ROPE>;
+    if (first_use_on_device((const void*)kern))
+        DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_split_smem<D>()));
+    const int gqa = p.Hq / p.Hkv, groups = (gqa + 8 * NH - 1) / (8 * NH);
+    DLP_CHECK_CUDA(launch_pdl(kern, dim3(p.n_splits, p.Hkv * groups, p.nq), dim3(128), attn_split_smem<D>(), s, p, ra));
     if (p.n_splits > 1 && p.counters == nullptr)
-        DLP_CHECK_CUDA(launch_pdl(attn_combine_kernel<D>, dim3(p.Hq, p.nq), dim3(D), 0, s, p));
+        DLP_CHECK_CUDA(launch_pdl(attn_combine_kernel<D>, dim3(p.Hq, p.nq), dim3(32), 0, s, p));
     return 0;
+}
+template <int D, bool ROPE>
+static int launch_attn(const AttnParams& p, const AttnRope& ra, cudaStream_t s) {
+    return p.Hq / p.Hkv <= 8 ? launch_attn_split<D, 1, ROPE>(p, ra, s) : launch_attn_split<D, 2, ROPE>(p, ra, s);
+}
+
+// The one-launch form for long contexts: RoPE, K / V write and split-KV attention with the splits joined through the caller's workspace.
+int attn_decode_split(const AttnParams& p_in, const float* qkv, const float* inv_freq, const float2* rope_cs, __half* kc_w, __half* vc_w, int D,
+                      int neox, float q_scale, cudaStream_t s) {
+    AttnParams p = p_in;
+    p.trace = trace_buffer();
+    p.pdl_early = attn_pdl_early();
+    DLP_REQUIRE(inv_freq != nullptr || rope_cs != nullptr, "attn_decode_split: need inv_freq or a (cos, sin) table");
+    DLP_REQUIRE(p.nq > 0 && p.Hq % p.Hkv == 0, "attn_decode_split: bad head configuration Hq=%d Hkv=%d", p.Hq, p.Hkv);
+    DLP_REQUIRE(p.n_splits >= 1 && (p.n_splits == 1 || (p.part_o && p.part_ml && p.counters)), "attn_decode_split: split-KV needs a workspace");
+    const AttnRope ra = {qkv, inv_freq, rope_cs, kc_w, vc_w, neox, q_scale};
+    if (D == 64) return launch_attn<64, true>(p, ra, s);
+    if (D == 128) return launch_attn<128, true>(p, ra, s);
+    DLP_REQUIRE(false, "attn_decode_split: head dim %d unsupported (64, 128)", D);
 }
 
 int attn_paged(const AttnParams& p_in, int D, cudaStream_t s) {
@@ -586,8 +812,9 @@ int attn_paged(const AttnParams& p_in, int D, cudaStream_t s) {
     p.trace = trace_buffer();
     DLP_REQUIRE(p.nq > 0 && p.Hq % p.Hkv == 0, "attn: bad head configuration Hq=%d Hkv=%d", p.Hq, p.Hkv);
     DLP_REQUIRE(p.n_splits >= 1 && (p.n_splits == 1 || (p.part_o && p.part_ml)), "attn: split-KV needs a workspace");
-    if (D == 64) return launch_attn<64>(p, s);
-    if (D == 128) return launch_attn<128>(p, s);
+    const AttnRope none = {};
+    if (D == 64) return launch_attn<64, false>(p, none, s);
+    if (D == 128) return launch_attn<128, false>(p, none, s);
     DLP_REQUIRE(false, "attn: head dim %d unsupported (64, 128)", D);
 }
 
@@ -604,24 +831,6 @@ int attn_paged(const AttnParams& p_in, int D, cudaStream_t s) {
 // planned upgrade.
 namespace dlp {
 
-
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem)));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem)));
-}
-__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
-    __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
 
 template <int D>
 __global__ void __launch_bounds__(128) attn_prefill_kernel(const __half* __restrict__ q, const __half* __restrict__ kc,

@@ -300,6 +300,19 @@ int dlp_attn_decode_rope(const float* qkv, const float* inv_freq, const float* r
                             (cudaStream_t)stream);
 }
 
+int dlp_attn_decode_split(const float* qkv, const float* inv_freq, const float* rope_cs, void* k_cache, void* v_cache, const int32_t* block_table,
+                          const int32_t* bt_row, const int32_t* kv_len, void* out, float* part_o, float* part_ml, int32_t* counters, int nq, int Hq,
+                          int Hkv, int D, int max_pages, int page_size, int n_splits, int neox, float q_scale, void* stream) {
+    DLP_REQUIRE(qkv && (inv_freq || rope_cs) && k_cache && v_cache && block_table && kv_len && out, "dlp_attn_decode_split: null argument");
+    DLP_REQUIRE(((uintptr_t)rope_cs & 7) == 0 && ((uintptr_t)qkv & 7) == 0, "dlp_attn_decode_split: qkv / rope_cs must be 8-byte aligned");
+    AttnParams p;
+    p.q = nullptr; p.kc = (const __half*)k_cache; p.vc = (const __half*)v_cache;
+    p.block_table = block_table; p.bt_row = bt_row; p.kv_len = kv_len; p.out = (__half*)out;
+    p.part_o = part_o; p.part_ml = part_ml; p.counters = counters;
+    p.nq = nq; p.Hq = Hq; p.Hkv = Hkv; p.max_pages = max_pages; p.page_size = page_size; p.n_splits = n_splits;
+    return attn_decode_split(p, qkv, inv_freq, (const float2*)rope_cs, (__half*)k_cache, (__half*)v_cache, D, neox, q_scale, (cudaStream_t)stream);
+}
+
 int dlp_attn_paged_static(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table,
                           const int32_t* bt_row, const int32_t* kv_len, void* out, int nq, int Hq, int Hkv, int D,
                           int max_pages, int page_size, int n_splits, void* stream) {

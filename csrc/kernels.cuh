@@ -184,6 +184,8 @@ int f32_to_f16(const float* in, __half* out, size_t n, cudaStream_t s);
 int attn_paged(const AttnParams& p, int D, cudaStream_t s);
 int attn_paged_static(AttnParams p, int D, cudaStream_t s);
 // decode step in one launch: RoPE(Q, new K) + paged K/V write + split-KV attention + cluster/DSMEM combine (attention.cu)
+int attn_decode_split(const AttnParams& p, const float* qkv, const float* inv_freq, const float2* rope_cs, __half* kc_w, __half* vc_w, int D,
+                      int neox, float q_scale, cudaStream_t s);
 int attn_decode_rope(const AttnParams& p, const float* qkv, const float* inv_freq, const float2* rope_cs, __half* kc_w,
                      __half* vc_w, int D, int neox, float q_scale, cudaStream_t s);
 int advance_rope(int* seq_len, const int* active, int* pos, int* slot, int* kv_len, const int* block_table, int max_pages,

@@ -83,33 +83,36 @@ class LlamaEngine(EngineCore):
         self.logits = torch.zeros(max(max_seqs, 1), v1 - v0, dtype=f32, device=dev) if last_stage else None
         if last_stage and self.comm.tp_size > 1 and hasattr(self.comm, "reserve_logits") and (v1 - v0) != cfg.vocab_size:
             self.comm.reserve_logits(max_seqs, v1 - v0, f32, dev)     # before any graph is captured
-        self.attn_splits = attn_splits if attn_splits is not None else (16 if dev.type == "cuda" else 1)
-        ns = self.attn_splits
-        self.attn_ws = (torch.zeros(max_seqs * self.Hq * ns * self.D, dtype=f32, device=dev),
-                        torch.zeros(max_seqs * self.Hq * ns * 2, dtype=f32, device=dev),
-                        torch.zeros(max_seqs * self.Hq, dtype=i32, device=dev)) if ns > 1 else None
+        # splits of the cached keys by batch size (index: queries of the step)
+        n_sm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 0
+        self.attn_splits = [0] + [attn_splits if attn_splits is not None else ops.attn_splits(b, self.Hkv, self.Hq // self.Hkv, n_sm) if n_sm else 1
+                                  for b in range(1, max_seqs + 1)]
+        parts = max(b * ns for b, ns in enumerate(self.attn_splits)) * self.Hq
+        self.attn_ws = (torch.zeros(parts * self.D, dtype=f32, device=dev), torch.zeros(parts * 2, dtype=f32, device=dev),
+                        torch.zeros(max_seqs * self.Hq, dtype=i32, device=dev)) if max(self.attn_splits) > 1 else None
         self.scratch = None  # fp16 decode buffer for block-quantised weights on the GEMM path (allocated lazily)
-        # decode attention in one launch (RoPE + KV write + split-KV + cluster combine); plain-llama layers with full-width RoPE
+        # decode attention in one launch (RoPE + KV write + split-KV + join of the splits); plain-llama layers with full-width RoPE
         self.attn_onepass = (dev.type == "cuda" and os.environ.get("DLP_ATTN_ONEPASS", "1") == "1" and cfg.rope_dim == self.D
                              and not cfg.qkv_bias and not cfg.qk_norm)
         self.attn_cluster = int(os.environ.get("DLP_ATTN_CLUSTER", "16"))
-        # the cluster launch only pays once the context spans more than one 64-key split; below this many keys the two-kernel
-        # path (RoPE kernel + attention) is used (profiles/r1_attn_onepass_ab.txt).  The host knows every sequence length, so the choice is part of the graph key.
-        self.attn_onepass_min = int(os.environ.get("DLP_ATTN_ONEPASS_MIN", "64"))
+        # below this many keys the two-kernel path (RoPE kernel + attention) is used: never, unless asked for (64 keys: 3.4 us in one launch,
+        # 2.6 + 3.4 in two).  The host knows every sequence length, so the choice is part of the graph key.
+        self.attn_onepass_min = int(os.environ.get("DLP_ATTN_ONEPASS_MIN", "1"))
         self._variant = False
         self.rope_cs = (torch.zeros(max_seqs, self.D // 2, 2, dtype=f32, device=dev)
                         if self.attn_onepass and os.environ.get("DLP_ROPE_TABLE", "1") == "1" else None)
 
-    # the decode step has two attention variants (one-launch cluster kernel or RoPE + attention): `_variant` is True for the former
+    # attention variants of a decode step of up to 4 sequences: everything in one launch (True) or RoPE + attention (False); larger steps
+    # have the second only
     @property
     def _onepass_now(self) -> bool:
         return bool(self._variant)
 
     def _choose_variant(self, B: int, max_len: int):
-        self._variant = self.attn_onepass and max_len >= self.attn_onepass_min
+        self._variant = self.attn_onepass and B <= 4 and max_len >= self.attn_onepass_min
 
     def _companion_variants(self) -> list:
-        return [not self._variant] if self.attn_onepass else []
+        return [not self._variant] if self.attn_onepass and self.attn_onepass_min > 1 and len(self._active_host) <= 4 else []
 
     def _graph_ok(self) -> bool:
         moe_lw = next((lw for lw in self.w.layers.values() if lw.router is not None), None)
@@ -434,15 +437,16 @@ class LlamaEngine(EngineCore):
     # ---- attention flavours ---------------------------------------------------------------------
     def _attn_decode(self, il, q, T):
         return ops.attn_paged(q, self.kv.k[il], self.kv.v[il], self.kv.block_table, self.kv_len[:T], self.Hq, self.Hkv,
-                              self.D, bt_row=self.active[:T], n_splits=self.attn_splits, workspace=self.attn_ws,
+                              self.D, bt_row=self.active[:T], n_splits=self.attn_splits[T], workspace=self.attn_ws,
                               out=self.att[:T])
 
     def _attn_decode_onepass(self, il, qkv, T):
         rope_on = self.inv_freq_off is None or self.cfg.layer_uses_rope(il)     # off: no (cos, sin) table, angles from the zero table
         return ops.attn_decode_rope(qkv, self._inv_freq(il), self.kv.k[il], self.kv.v[il], self.kv.block_table, self.kv_len[:T],
-                                    self.Hq, self.Hkv, self.D, bt_row=self.active[:T], n_splits=self.attn_cluster,
+                                    self.Hq, self.Hkv, self.D, bt_row=self.active[:T], n_splits=self.attn_cluster if self.attn_ws is None else self.attn_splits[T],
                                     neox=self.cfg.rope_neox, attn_scale=self.attn_scale, out=self.att[:T],
-                                    rope_cs=self.rope_cs[:T] if (self.rope_cs is not None and rope_on) else None)
+                                    rope_cs=self.rope_cs[:T] if (self.rope_cs is not None and rope_on) else None,
+                                    workspace=self.attn_ws)
 
     def _attn_prefill_for(self, sid: int, pos0: int):
         def fn(il, q, T):

@@ -287,6 +287,15 @@ def _attn_cpu(q, k_cache, v_cache, block_table_rows, kv_len, n_head, n_head_kv, 
     return out
 
 
+def attn_splits(nq: int, n_head_kv: int, group: int, n_sm: int) -> int:
+    """Key splits of a decode attention launch (a cap: the kernel takes one per 256 keys of each query's own length).  One query: one full
+    wave of the kernel's two CTAs an SM (32,000 keys of 8 KV heads: 28.7 us with 37 splits, 32.1 with 16, 35.1 with 74).  Several: two waves,
+    because their lengths differ; a split that a short query does not need returns at once, but still has to be started (32 queries of up to
+    2,000 keys: 33 to 37 us with 2 to 4 splits, 43 with 8, 52 with 16; of up to 300: 13 us with 2, 16 with 8)."""
+    pairs = nq * n_head_kv * ((group + 15) // 16)
+    return max(1, 2 * n_sm // pairs) if nq == 1 else max(1, (4 * n_sm + pairs - 1) // pairs)
+
+
 def attn_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                kv_len: torch.Tensor, n_head: int, n_head_kv: int, head_dim: int, bt_row: torch.Tensor | None = None,
                n_splits: int = 1, workspace: tuple[torch.Tensor, torch.Tensor] | None = None,
@@ -329,9 +338,11 @@ def attn_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, bl
 def attn_decode_rope(qkv: torch.Tensor, inv_freq: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                      block_table: torch.Tensor, kv_len: torch.Tensor, n_head: int, n_head_kv: int, head_dim: int,
                      bt_row: torch.Tensor | None = None, n_splits: int = 8, neox: bool = False, attn_scale: float = 1.0,
-                     out: torch.Tensor | None = None, rope_cs: torch.Tensor | None = None) -> torch.Tensor:
+                     out: torch.Tensor | None = None, rope_cs: torch.Tensor | None = None,
+                     workspace: tuple[torch.Tensor, torch.Tensor, torch.Tensor] | None = None) -> torch.Tensor:
     """One-launch decode attention: RoPE on Q and the new K, K/V page write at position kv_len-1, split-KV attention with the
-    splits combined inside a thread-block cluster.  qkv: fp32 [nq, (Hq+2Hkv)*D] straight from the QKV mat-vec."""
+    splits (up to 16) combined inside a thread-block cluster, or with a `workspace` (partials, lse, counters: as for attn_paged) any number
+    of them joined through it (long contexts).  qkv: fp32 [nq, (Hq+2Hkv)*D] straight from the QKV mat-vec."""
     nq = qkv.shape[0]
     if out is None:
         out = torch.empty(nq, n_head * head_dim, dtype=torch.float16, device=qkv.device)
@@ -343,6 +354,14 @@ def attn_decode_rope(qkv: torch.Tensor, inv_freq: torch.Tensor, k_cache: torch.T
         slot = (page * ps + pos % ps).to(torch.int32)
         q = rope_kv(qkv, pos, slot, inv_freq, k_cache, v_cache, n_head, n_head_kv, head_dim, neox, attn_scale=attn_scale)
         return attn_paged(q, k_cache, v_cache, block_table, kv_len, n_head, n_head_kv, head_dim, bt_row=bt_row, out=out)
+    if workspace is not None:
+        po, pm, ctr = workspace
+        _lib.check(_lib.load().dlp_attn_decode_split(
+            qkv.data_ptr(), inv_freq.data_ptr(), _p(rope_cs), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(), _p(bt_row),
+            kv_len.data_ptr(), out.data_ptr(), po.data_ptr(), pm.data_ptr(), ctr.data_ptr(), nq, n_head, n_head_kv, head_dim,
+            block_table.shape[1], k_cache.shape[2], n_splits, int(neox), attn_scale / math.sqrt(head_dim), _stream()), "attn_decode_split")
+        _count()
+        return out
     _lib.check(_lib.load().dlp_attn_decode_rope(
         qkv.data_ptr(), inv_freq.data_ptr(), _p(rope_cs), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(), _p(bt_row),
         kv_len.data_ptr(), out.data_ptr(), nq, n_head, n_head_kv, head_dim, block_table.shape[1], k_cache.shape[2],

@@ -68,6 +68,7 @@ def _declare(lib):
         "dlp_attn_paged_fused": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]),
         "dlp_set_trace": (i32, [vp]),
         "dlp_advance_rope": (i32, [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp, i32, vp, vp]),
+        "dlp_attn_decode_split": (i32, [vp] * 12 + [i32] * 8 + [f32, vp]),
         "dlp_attn_decode_rope": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp]),
         "dlp_attn_prefill": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]),
         "dlp_argmax": (i32, [vp, i32, i32, i32, vp, vp]),

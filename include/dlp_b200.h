@@ -124,8 +124,8 @@ int dlp_attn_paged(const void* q, const void* k_cache, const void* v_cache, cons
                    const int32_t* bt_row, const int32_t* kv_len, void* out, float* part_o, float* part_ml, int nq,
                    int Hq, int Hkv, int D, int max_pages, int page_size, int n_splits, void* stream);
 
-/* Same, with the split-KV combine fused into the attention kernel: `counters` is an int32 array of nq * Hkv * (Hq/Hkv/G)
- * entries (G = 4, 2 or 1 query heads per CTA; nq * Hq entries always suffice), zero-initialised once; the last split CTA of
+/* Same, with the split-KV combine fused into the attention kernel: `counters` is an int32 array of nq * Hq
+ * entries (one per query and group of query heads is used), zero-initialised once; the last split CTA of
  * each (query, kv-head group) merges the partials and resets its counter.  One launch instead of two. */
 int dlp_attn_paged_fused(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table,
                          const int32_t* bt_row, const int32_t* kv_len, void* out, float* part_o, float* part_ml,
@@ -150,6 +150,12 @@ int dlp_advance_rope(int32_t* seq_len, const int32_t* active, int32_t* pos, int3
 int dlp_attn_decode_rope(const float* qkv, const float* inv_freq, const float* rope_cs, void* k_cache, void* v_cache, const int32_t* block_table,
                          const int32_t* bt_row, const int32_t* kv_len, void* out, int nq, int Hq, int Hkv, int D, int max_pages,
                          int page_size, int n_splits, int neox, float q_scale, void* stream);
+
+/* The same step, faster where a workspace is at hand: any number of splits, joined through the workspace of dlp_attn_paged_fused (part_o, part_ml, counters) by
+ * the last CTA to finish.  The arguments and the ordering rule of dlp_attn_decode_rope hold. */
+int dlp_attn_decode_split(const float* qkv, const float* inv_freq, const float* rope_cs, void* k_cache, void* v_cache, const int32_t* block_table,
+                          const int32_t* bt_row, const int32_t* kv_len, void* out, float* part_o, float* part_ml, int32_t* counters, int nq, int Hq,
+                          int Hkv, int D, int max_pages, int page_size, int n_splits, int neox, float q_scale, void* stream);
 
 /* dlp_attn_paged for callers that cannot supply the split-KV workspace.  (No counterpart in the reference: it always
  * allocates its own split buffers from the backend pool.)

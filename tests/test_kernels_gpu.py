@@ -310,6 +310,46 @@ def test_attn_decode_rope_onepass(D, Hq, Hkv, neox, n_splits):
     assert torch.equal(kc.cpu()[untouched], kc_ref[untouched])          # nothing else in the cache was written
 
 
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 8, 2), (64, 16, 2), (128, 24, 2), (64, 40, 2)])      # 4, 8, 12 and 20 query heads to a key head
+@pytest.mark.parametrize("page", [16, 64])
+@pytest.mark.parametrize("n_splits", [1, 3, 40])
+def test_attn_split_tiles_and_joins(D, Hq, Hkv, page, n_splits):
+    """Split-KV attention at the edges of its tiles (16 keys), warps (4 tiles) and splits (256 keys), with and without RoPE and the new token's
+    K / V in the same launch, against 64 bits.  Bound: the output is rounded to fp16 (relative 2^-12 on average, squared 6e-8)."""
+    lens = [1, 15, 16, 17, 64, 65, 256, 257, 511, 513, 1040, 3001]
+    nq, per = len(lens), (max(lens) + page - 1) // page
+    kc, vc = _fill_cache(nq * per, Hkv, page, D, seed=5)
+    bt = torch.randperm(nq * per, generator=torch.Generator().manual_seed(1)).view(nq, per).to(torch.int32).to(DEV)
+    kv_len = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    qkv = torch.randn(nq, (Hq + 2 * Hkv) * D, device=DEV, generator=torch.Generator(DEV).manual_seed(2))
+    inv = (10000.0 ** (-torch.arange(0, D // 2).double() * 2 / D)).float().to(DEV)
+    ws = (torch.full((nq * Hq * n_splits * D,), math.nan, device=DEV), torch.full((nq * Hq * n_splits * 2,), math.nan, device=DEV),
+          torch.zeros(nq * Hq, dtype=torch.int32, device=DEV))
+
+    def exact(q, i, n):
+        pg = bt[i, :(n + page - 1) // page].long()
+        k, v = (c[pg].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :n].double().repeat_interleave(Hq // Hkv, 0) for c in (kc, vc))
+        return (torch.softmax(k @ q.view(Hq, D, 1).double(), 1) * v).sum(1).view(-1)
+    for neox in (False, True):
+        out = ops.attn_decode_rope(qkv, inv, kc, vc, bt, kv_len, Hq, Hkv, D, n_splits=n_splits, neox=neox, workspace=ws)
+        x = qkv.double().view(nq, -1, D)
+        for i, n in enumerate(lens):
+            a = (n - 1) * inv.double()
+            rot = x[i, :Hq + Hkv]
+            u, v = (rot[:, :D // 2], rot[:, D // 2:]) if neox else (rot[:, 0::2], rot[:, 1::2])
+            pair = (u * a.cos() - v * a.sin(), u * a.sin() + v * a.cos())
+            rot = torch.cat(pair, -1) if neox else torch.stack(pair, -1).flatten(-2)
+            row = (bt[i, (n - 1) // page].long(), slice(None), (n - 1) % page)
+            assert nmse(rot[Hq:], kc[row]) < 1e-6 and torch.equal(x[i, Hq + Hkv:].half(), vc[row])
+            assert nmse(exact(rot[:Hq] * D ** -0.5, i, n), out[i]) < 2e-7, (neox, n)
+    q = (torch.randn(nq, Hq * D, device=DEV) / math.sqrt(D)).half()
+    joined = ops.attn_paged(q, kc, vc, bt, kv_len, Hq, Hkv, D, n_splits=n_splits, workspace=ws)
+    assert torch.equal(joined, ops.attn_paged(q, kc, vc, bt, kv_len, Hq, Hkv, D, n_splits=n_splits))
+    for i, n in enumerate(lens):
+        assert nmse(exact(q[i], i, n), joined[i]) < 2e-7, n
+    assert int(ws[2].abs().sum()) == 0
+
+
 @pytest.mark.parametrize("impl", ["tc", "mma"])
 @pytest.mark.parametrize("D,Hq,Hkv", [(128, 8, 2), (64, 4, 2)])
 @pytest.mark.parametrize("T,pos0,page", [(5, 0, 16), (64, 0, 16), (100, 37, 16), (200, 64, 16), (128, 0, 64), (300, 250, 64), (513, 1000, 64), (1, 400, 8)])
