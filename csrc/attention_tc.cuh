@@ -183,7 +183,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
     if (warp == 0) {
         // ===== producer =====
-        if (lane == 0) {
+        if (elect_one()) {      // (elect.sync: with lane == 0 the compiler issues TMA and MMAs through a loop over the lanes, 100 clocks each)
             mbar_expect_tx(q_full, Cfg::Q_BYTES);
             for (int kb = 0; kb < KB; ++kb) tma_load_2d(sm_q + kb * (BM * 128), &tm_q, q_full, hq * (MODE == FA_TILES ? p.q_head : D1) + kb * 64, t0);
             const int ps = MODE == FA_ROWS ? BN : p.page_size, chunks = BN / ps;
@@ -214,7 +214,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = make_idesc_f16(BM, BN, FMT);
             constexpr uint32_t idesc_o = make_idesc_f16_bmn(BM, D2, FMT);
             auto issue_pv = [&](int j) {

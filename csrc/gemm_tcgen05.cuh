@@ -56,6 +56,28 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x))
 // tanh form of gelu: 0.5 (1 + tanh u) is the sigmoid of 2u
 __device__ __forceinline__ float gelu_f(float x) { return x / (1.f + __expf(-1.5957691216057308f * (x + 0.044715f * x * x * x))); }
 
+static __device__ int g_gemm_wait_expired;      // a bounded wait ran into its limit (dlp_gemm_wait_expired)
+
+// After the limit the flag is set and every later wait gives up after a short try, so the kernel runs to its end, frees its tensor memory
+// and returns (with wrong results).
+template <bool CLUSTER = false>
+__device__ __forceinline__ void mbar_wait_b(uint64_t* bar, uint32_t parity) {
+    for (unsigned spins = 0; !(CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)); ++spins) {
+        if ((spins & 1023u) == 1023u && *reinterpret_cast<volatile int*>(&g_gemm_wait_expired) != 0) return;
+        if (spins > (1u << 22)) { atomicExch(&g_gemm_wait_expired, 1); return; }
+    }
+}
+static inline int gemm_wait_flag(int* out) {      // this translation unit's flag (current device)
+    int v = 0;
+    DLP_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_gemm_wait_expired, sizeof(int)));
+    *out |= v;
+    return 0;
+}
+__device__ __forceinline__ void gemm_wait_aftermath() {
+    if (threadIdx.x == 0 && *reinterpret_cast<volatile int*>(&g_gemm_wait_expired) != 0)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);       // a wait gave up: copies in flight land before the block goes away
+}
+
 // ---- dequant-fused A operand ---------------------------------------------------------------------------
 // For block-quantised weights the four epilogue warps (idle while the accumulator is being built) act as the
 // A-operand producer: thread r owns row r of the 128-row tile, decodes that row's 64-element K slice from
@@ -160,6 +182,115 @@ __device__ __forceinline__ void epi_loop(const GemmParams& p, const uint32_t (&r
     }
 }
 
+// Epilogue of one 128 x BT tile by 4 warps (threads 64 .. 191 of the block): accumulators -> y, or with split-K through the workspace
+template <int BT, int NA, int AB_FMT>
+__device__ __forceinline__ void gemm_drain(const GemmParams& p, uint32_t tmem_base, uint64_t* tmem_full_bar, bool any, int n_out0, int t0, int t_end) {
+    // warp%4 selects the TMEM lane quarter
+    const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3;
+    const int n_local = q * 32 + lane;
+    const int n = n_out0 + n_local;
+    const float bias = p.epilogue == EPI_TAIL_BF16 && p.tail.bias != nullptr && n < p.N ? p.tail.bias[n] : 0.f;      // (requested before the accumulators are there)
+    if (any) {
+        mbar_wait(tmem_full_bar, 0);
+        tc_fence_after();
+    }
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    constexpr int CH = BT >= 32 ? 32 : 16;
+    const int S = gridDim.z;
+    const bool split_ws = p.ws != nullptr && S > 1;
+    const size_t tile = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    auto load_acc = [&](int c, uint32_t (&r0)[CH], uint32_t (&r1)[CH]) {
+        if (any) {
+            if constexpr (CH == 32) {
+                tmem_ld_32x32(lane_addr + c * CH, r0);
+                if (NA == 2) tmem_ld_32x32(lane_addr + BT + c * CH, r1);
+            } else {
+                tmem_ld_32x16(lane_addr + c * CH, r0);
+                if (NA == 2) tmem_ld_32x16(lane_addr + BT + c * CH, r1);
+            }
+            tc_wait_ld();
+        } else {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) { r0[j] = 0; r1[j] = 0; }
+        }
+    };
+    auto run_epilogue = [&](int c, const uint32_t (&r0)[CH], const uint32_t (&r1)[CH]) {
+        if (n < p.N) {
+            // one specialised store loop per epilogue (dispatch hoisted out of the per-element loop: a switch with the
+            // reduce-scatter address arithmetic inside it cost 35-50 % of the whole GEMM, see profiles/r1_gemm_ab.txt)
+            const int tb = t0 + c * CH;
+            switch (p.epilogue) {
+                case EPI_STORE_F16: epi_loop<EPI_STORE_F16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_STORE_BF16: epi_loop<EPI_STORE_BF16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_STORE_F32: epi_loop<EPI_STORE_F32, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_ATOMIC_ADD_F32: epi_loop<EPI_ATOMIC_ADD_F32, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_SWIGLU_F16: if (NA == 2) epi_loop<EPI_SWIGLU_F16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_GEGLU_BF16: if (NA == 2 && AB_FMT == 1) epi_loop<EPI_GEGLU_BF16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_SWIGLU_BF16: if (NA == 2 && AB_FMT == 1) epi_loop<EPI_SWIGLU_BF16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_RELU2_BF16: if (NA == 1 && AB_FMT == 1) epi_loop<EPI_RELU2_BF16, CH>(p, r0, r1, tb, n, t_end); break;
+                case EPI_TAIL_BF16: if (NA == 1 && AB_FMT == 1) epi_loop<EPI_TAIL_BF16, CH>(p, r0, r1, tb, n, t_end, bias); break;
+                case EPI_RS_PUSH_F32: epi_loop<EPI_RS_PUSH_F32, CH>(p, r0, r1, tb, n, t_end); break;
+            }
+        }
+    };
+    if (!split_ws) {
+#pragma unroll 1
+        for (int c = 0; c < BT / CH; ++c) {
+            if (t0 + c * CH >= t_end) break;  // warp-uniform
+            uint32_t r0[CH], r1[CH];
+            load_acc(c, r0, r1);
+            run_epilogue(c, r0, r1);
+        }
+    } else {
+        // partial tile -> workspace [tile][split][accumulator][token][128 features] (128 consecutive floats per store round)
+        __shared__ int s_last;
+        float* wsp = p.ws + ((tile * S + blockIdx.z) * NA) * (size_t)BT * GEMM_BM;
+#pragma unroll 1
+        for (int c = 0; c < BT / CH; ++c) {
+            if (t0 + c * CH >= t_end) break;
+            uint32_t r0[CH], r1[CH];
+            load_acc(c, r0, r1);
+#pragma unroll
+            for (int j = 0; j < CH; ++j) {
+                __stcg(wsp + (size_t)(c * CH + j) * GEMM_BM + n_local, __uint_as_float(r0[j]));
+                if (NA == 2) __stcg(wsp + (size_t)(BT + c * CH + j) * GEMM_BM + n_local, __uint_as_float(r1[j]));
+            }
+        }
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (threadIdx.x == 64) s_last = (atomicAdd(p.ws_counters + tile, 1u) == (unsigned)(S - 1)) ? 1 : 0;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (s_last) {
+            __threadfence();
+            const float* base = p.ws + (tile * S * NA) * (size_t)BT * GEMM_BM;
+#pragma unroll 1
+            for (int c = 0; c < BT / CH; ++c) {
+                if (t0 + c * CH >= t_end) break;
+                uint32_t r0[CH], r1[CH];
+#pragma unroll
+                for (int j = 0; j < CH; ++j) r0[j] = r1[j] = 0u;
+                for (int z = 0; z < S; ++z) {          // fixed order: the result does not depend on which split finished last
+                    const float* pz = base + (size_t)z * NA * BT * GEMM_BM + (size_t)(c * CH) * GEMM_BM + n_local;
+                    // all loads of a split in flight (splits innermost: a chain of S latencies per value, 24 of 27 us at 6 splits)
+                    float v0[CH], v1[CH];
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) {
+                        v0[j] = __ldcg(pz + (size_t)j * GEMM_BM);
+                        if (NA == 2) v1[j] = __ldcg(pz + (size_t)(BT + j) * GEMM_BM);
+                    }
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) {
+                        r0[j] = __float_as_uint(__uint_as_float(r0[j]) + v0[j]);
+                        if (NA == 2) r1[j] = __float_as_uint(__uint_as_float(r1[j]) + v1[j]);
+                    }
+                }
+                run_epilogue(c, r0, r1);
+            }
+            if (threadIdx.x == 64) p.ws_counters[tile] = 0;    // ready for the next launch
+        }
+    }
+}
+
 template <int BT, int NA, int AB_FMT, int WT>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
@@ -219,7 +350,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
 
     if (warp == 0) {
         // ===== TMA producer =====
-        if (lane == 0) {
+        if (elect_one()) {      // (elect.sync: with lane == 0 the compiler issues TMA and MMAs through a loop over the lanes, 100 clocks each)
             if (p.coll.x_flags != nullptr) {
                 // all-gather -> GEMM: the token rows of this tile were pushed into our gather buffer by their owner
                 // ranks; wait for exactly those owners, then order the acquired generic-proxy view before the TMA reads
@@ -251,7 +382,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         }
     } else if (warp == 1) {
         // ===== MMA issuer (one thread) =====
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc_f16(GEMM_BM, BT, AB_FMT);
             int stage = 0;
             uint32_t phase = 0;
@@ -292,104 +423,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
-        // ===== epilogue: 4 warps, warp%4 selects the TMEM lane quarter =====
-        const int q = warp & 3;
-        const int n_local = q * 32 + lane;
-        const int n = n_out0 + n_local;
-        const float bias = p.epilogue == EPI_TAIL_BF16 && p.tail.bias != nullptr && n < p.N ? p.tail.bias[n] : 0.f;      // (requested before the accumulators are there)
-        if (num_kb > 0) {
-            mbar_wait(tmem_full_bar, 0);
-            tc_fence_after();
-        }
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-        constexpr int CH = BT >= 32 ? 32 : 16;
-        const int S = gridDim.z;
-        const bool split_ws = p.ws != nullptr && S > 1;
-        const size_t tile = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
-        auto load_acc = [&](int c, uint32_t (&r0)[CH], uint32_t (&r1)[CH]) {
-            if (num_kb > 0) {
-                if constexpr (CH == 32) {
-                    tmem_ld_32x32(lane_addr + c * CH, r0);
-                    if (NA == 2) tmem_ld_32x32(lane_addr + BT + c * CH, r1);
-                } else {
-                    tmem_ld_32x16(lane_addr + c * CH, r0);
-                    if (NA == 2) tmem_ld_32x16(lane_addr + BT + c * CH, r1);
-                }
-                tc_wait_ld();
-            } else {
-#pragma unroll
-                for (int j = 0; j < CH; ++j) { r0[j] = 0; r1[j] = 0; }
-            }
-        };
-        auto run_epilogue = [&](int c, const uint32_t (&r0)[CH], const uint32_t (&r1)[CH]) {
-            if (n < p.N) {
-                // one specialised store loop per epilogue (dispatch hoisted out of the per-element loop: a switch with the
-                // reduce-scatter address arithmetic inside it cost 35-50 % of the whole GEMM, see profiles/r1_gemm_ab.txt)
-                const int tb = t0 + c * CH;
-                switch (p.epilogue) {
-                    case EPI_STORE_F16: epi_loop<EPI_STORE_F16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_STORE_BF16: epi_loop<EPI_STORE_BF16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_STORE_F32: epi_loop<EPI_STORE_F32, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_ATOMIC_ADD_F32: epi_loop<EPI_ATOMIC_ADD_F32, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_SWIGLU_F16: if (NA == 2) epi_loop<EPI_SWIGLU_F16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_GEGLU_BF16: if (NA == 2 && AB_FMT == 1) epi_loop<EPI_GEGLU_BF16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_SWIGLU_BF16: if (NA == 2 && AB_FMT == 1) epi_loop<EPI_SWIGLU_BF16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_RELU2_BF16: if (NA == 1 && AB_FMT == 1) epi_loop<EPI_RELU2_BF16, CH>(p, r0, r1, tb, n, t_end); break;
-                    case EPI_TAIL_BF16: if (NA == 1 && AB_FMT == 1) epi_loop<EPI_TAIL_BF16, CH>(p, r0, r1, tb, n, t_end, bias); break;
-                    case EPI_RS_PUSH_F32: epi_loop<EPI_RS_PUSH_F32, CH>(p, r0, r1, tb, n, t_end); break;
-                }
-            }
-        };
-        if (!split_ws) {
-#pragma unroll 1
-            for (int c = 0; c < BT / CH; ++c) {
-                if (t0 + c * CH >= t_end) break;  // warp-uniform
-                uint32_t r0[CH], r1[CH];
-                load_acc(c, r0, r1);
-                run_epilogue(c, r0, r1);
-            }
-        } else {
-            // partial tile -> workspace [tile][split][accumulator][token][128 features] (128 consecutive floats per store round)
-            __shared__ int s_last;
-            float* wsp = p.ws + ((tile * S + blockIdx.z) * NA) * (size_t)BT * GEMM_BM;
-#pragma unroll 1
-            for (int c = 0; c < BT / CH; ++c) {
-                if (t0 + c * CH >= t_end) break;
-                uint32_t r0[CH], r1[CH];
-                load_acc(c, r0, r1);
-#pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                    __stcg(wsp + (size_t)(c * CH + j) * GEMM_BM + n_local, __uint_as_float(r0[j]));
-                    if (NA == 2) __stcg(wsp + (size_t)(BT + c * CH + j) * GEMM_BM + n_local, __uint_as_float(r1[j]));
-                }
-            }
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (threadIdx.x == 64) s_last = (atomicAdd(p.ws_counters + tile, 1u) == (unsigned)(S - 1)) ? 1 : 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (s_last) {
-                __threadfence();
-                const float* base = p.ws + (tile * S * NA) * (size_t)BT * GEMM_BM;
-#pragma unroll 1
-                for (int c = 0; c < BT / CH; ++c) {
-                    if (t0 + c * CH >= t_end) break;
-                    uint32_t r0[CH], r1[CH];
-#pragma unroll
-                    for (int j = 0; j < CH; ++j) {
-                        float a0 = 0.f, a1 = 0.f;
-                        for (int z = 0; z < S; ++z) {      // fixed order: the result does not depend on which split finished last
-                            const float* pz = base + (size_t)z * NA * BT * GEMM_BM;
-                            a0 += __ldcg(pz + (size_t)(c * CH + j) * GEMM_BM + n_local);
-                            if (NA == 2) a1 += __ldcg(pz + (size_t)(BT + c * CH + j) * GEMM_BM + n_local);
-                        }
-                        r0[j] = __float_as_uint(a0);
-                        r1[j] = __float_as_uint(a1);
-                    }
-                    run_epilogue(c, r0, r1);
-                }
-                if (threadIdx.x == 64) p.ws_counters[tile] = 0;    // ready for the next launch
-            }
-        }
+        gemm_drain<BT, NA, AB_FMT>(p, tmem_base, tmem_full_bar, num_kb > 0, n_out0, t0, t_end);
     }
     tc_fence_before();
     __syncthreads();
