@@ -3,6 +3,9 @@
 
 namespace dlp {
 
+bool gemm_pair_takes(int T, const GemmGroup* grp);
+int gemm_pair(const GemmParams& p, const void* w0, const void* w1, int ldw, const void* x, int ldx, int is_bf16, int na, int split_k, cudaStream_t stream);
+
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -32,6 +35,22 @@ int make_tmap_2d(CUtensorMap* out, const void* base, int is_bf16, uint64_t rows,
     CUresult r = enc(out, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    DLP_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+    return 0;
+}
+
+// 2-D map of bytes: box_bytes x 128 rows, swizzle of 0, 64 or 128 bytes
+int make_tmap_bytes(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_bytes, int swizzle) {
+    PFN_encodeTiled enc = get_encode_fn();
+    DLP_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled entry point unavailable (no CUDA driver?)");
+    DLP_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0 && row_bytes % 16 == 0, "TMA base pointer and row stride must be multiples of 16 bytes");
+    cuuint64_t dims[2] = {row_bytes, rows};
+    cuuint64_t strides[1] = {row_bytes};
+    cuuint32_t box[2] = {box_bytes, GEMM_BM};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     DLP_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return 0;
 }
@@ -71,6 +90,7 @@ int gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, vo
                 "gemm: the reduce-scatter epilogue needs a collective descriptor and no atomic split-K");
     p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue;
     if (grp) p.grp = *grp;
+    if (coll == nullptr && split_k <= 1 && gemm_pair_takes(T, grp)) return gemm_pair(p, w0, w1, ldw, x, ldx, is_bf16, na, split_k, stream);
     const int bt = grp ? grp->bt : (T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256);
     if (splits == 1)
         splits = auto_split_ws(epilogue, split_k, (long)((N + GEMM_BM - 1) / GEMM_BM) * (grp ? grp->max_tiles : (T + bt - 1) / bt), total_kb, na, bt,

@@ -123,6 +123,25 @@ def test_gemm_tcgen05_ragged_n_splitk_swiglu():
     assert nmse(torch.nn.functional.silu(ref) * (x.float() @ u.float().T), sw) < 5e-6
 
 
+@pytest.mark.parametrize("T,N,K", [(65, 256, 64), (100, 130, 200), (128, 300, 1024), (257, 512, 2056), (700, 4096, 512), (1030, 2304, 320)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gemm_on_pairs_of_sms(T, N, K, dtype):
+    """The smallest and widest token tiles, row tiles that end inside a pair or inside its second block, columns that are no multiple of 64, one and
+    several waves, with every kind of epilogue.  Sums are fp32 (relative 2^-24 sqrt(K)); 16-bit outputs round once more."""
+    g = torch.Generator(DEV).manual_seed(7)
+    x, w, u = ((torch.randn(n, K, device=DEV, generator=g) * s).to(dtype) for n, s in ((T, 1.0), (N, K ** -0.5), (N, K ** -0.5)))
+    ref, up = (x.double() @ m.double().T for m in (w, u))
+    y, acc = torch.zeros(T, N, device=DEV), torch.ones(T, N, device=DEV)
+    assert nmse(ref, ops.gemm_f16(w, x, y, epilogue=1)) < 1e-11
+    assert nmse(ref + 1, ops.gemm_f16(w, x, acc, epilogue=2)) < 1e-11
+    assert nmse(ref, ops.gemm_f16(w, x, torch.zeros(T, N, device=DEV, dtype=torch.float16), epilogue=0)) < 1e-7
+    assert nmse(torch.nn.functional.silu(ref) * up, ops.gemm_f16(w, x, torch.zeros(T, N, device=DEV, dtype=torch.float16), epilogue=3, w_up=u)) < 2e-7
+    if dtype == torch.bfloat16:
+        for epi, want in ((4, ref), (6, torch.nn.functional.gelu(ref, approximate="tanh") * up), (7, torch.relu(ref) ** 2), (8, torch.nn.functional.silu(ref) * up)):
+            out = ops.gemm_f16(w, x, torch.zeros(T, N, device=DEV, dtype=torch.bfloat16), epilogue=epi, w_up=u if epi in (6, 8) else None)
+            assert nmse(want, out) < 6e-6, epi
+
+
 @pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
 @pytest.mark.parametrize("T,N,K", [(48, 256, 512), (300, 200, 1024), (7, 384, 2048)])
 def test_linear_quant_dequant_fused_gemm(t, T, N, K):
