@@ -3,6 +3,10 @@
 
 namespace dlp {
 
+bool gemm_quant_small_takes(const QWeight& w, int wtype);
+int gemm_quant_small(const QWeight& w0, const QWeight& w1, int na, int wtype, int bt, const CUtensorMap& tx, const GemmParams& p, int split_k, void* ws,
+                     size_t ws_bytes, cudaStream_t stream);
+
 // Y[T,N] (op)= X[T,K] . dequant(W)[N,K]^T with the block-quant decode fused into the A-operand producer.
 int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, int ldx, void* y, int ldy, int T, int epilogue,
                int split_k, cudaStream_t stream, const GemmCollective* coll, const GemmGroup* grp, void* ws, size_t ws_bytes) {
@@ -35,6 +39,14 @@ int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, i
     p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue;
     if (grp) p.grp = *grp;
     const int bt = grp ? grp->bt : (T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256);
+    const QWeight up = w1 ? *w1 : QWeight();
+    // Token tiles of up to 64 stream the weights' bytes (gemm_quant_small.cuh); wider ones are bound by the MMAs.  At 64 tokens the
+    // bytes still bound it (Q8_0 gate and up of Llama-8B: 35 us, 7 tokens 34), at 128 one pass of gemm_tcgen05_kernel does the work of two of these.
+    if (bt <= 64 && coll == nullptr && epilogue != EPI_RS_PUSH_F32 && gemm_quant_small_takes(w0, wtype) && (na == 1 || gemm_quant_small_takes(up, wtype))) {
+        CUtensorMap tx;
+        if (int rc = make_tmap_2d(&tx, x, 0, T, K, ldx, bt)) return rc;
+        return gemm_quant_small(w0, up, na, wtype, bt, tx, p, split_k, ws, ws_bytes, stream);
+    }
     if (splits == 1)
         splits = auto_split_ws(epilogue, split_k, (long)((N + GEMM_BM - 1) / GEMM_BM) * (grp ? grp->max_tiles : (T + bt - 1) / bt), total_kb, na, bt,
                                ws, ws_bytes, p);
@@ -44,7 +56,6 @@ int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, i
     CUtensorMap tx;
     int rc;
     if ((rc = make_tmap_2d(&tx, x, 0, T, K, ldx, bt))) return rc;
-    const QWeight up = w1 ? *w1 : QWeight();
 #define DLP_QG_BT(WT_, BT_)                                                                                   \
     case BT_:                                                                                                 \
         return na == 2 ? launch_gemm<BT_, 2, 0, WT_>(tx, tx, tx, p, splits, stream, w0, up)                   \

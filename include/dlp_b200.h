@@ -116,6 +116,10 @@ int dlp_swiglu(const void* gate_up, int is_f16, void* out_f16, int T, int F, int
 int dlp_advance(int32_t* seq_len, const int32_t* active, int32_t* pos, int32_t* slot, int32_t* kv_len,
                 const int32_t* block_table, int max_pages, int page_size, int n, void* stream);
 
+/* *out = 1 when a wait inside one of the tensor-core kernels has run into its limit on the current device since the library was loaded (it then
+ * returned with wrong results instead of spinning on), else 0.  Synchronises with the device. */
+int dlp_gemm_wait_expired(int* out);
+
 /* Paged attention for nq queries (decode, batched decode, or one query per prefill token).
  * q/out fp16 [nq,Hq,D]; kv_len[q] keys visible; bt_row[q] selects the block-table row (NULL: q).
  * n_splits>1 uses split-KV with workspace part_o [nq*Hq*n_splits*D] / part_ml [nq*Hq*n_splits*2] floats.

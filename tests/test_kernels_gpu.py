@@ -159,6 +159,22 @@ def test_linear_quant_dequant_fused_gemm(t, T, N, K):
     assert nmse(torch.nn.functional.silu(ref) * (x.float() @ exact_u.T), sw) < 2e-5
 
 
+@pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
+@pytest.mark.parametrize("T,N,K", [(5, 128, 256), (16, 200, 512), (17, 126, 768), (33, 384, 2304), (64, 130, 4096), (65, 256, 512)])
+def test_linear_quant_few_tokens(t, T, N, K):
+    """Token tiles of 16, 32 and 64 (and the first size behind them), partial row tiles, one unit of columns up to several splits of K.  The weights
+    enter as fp16 values (relative 2^-12 on average, squared 2e-8 with the margin of the few that round the other way); sums are fp32."""
+    w, exact = _w(N, K, t, 1)
+    u, exact_u = _w(N, K, t, 2)
+    x = torch.randn(T, K, device=DEV, generator=torch.Generator(DEV).manual_seed(3)).half()
+    ref = x.double() @ exact.double().T
+    assert nmse(ref, ops.linear(w, x, "f32")) < 2e-7
+    acc = torch.ones(T, N, device=DEV)
+    assert nmse(ref + 1, ops.linear(w, x, "add", out=acc)) < 2e-7
+    assert nmse(ref, ops.linear(w, x, "f16")) < 4e-7          # (and the rounding of the output)
+    assert nmse(torch.nn.functional.silu(ref) * (x.double() @ exact_u.double().T), ops.linear(w, x, "swiglu", w_up=u)) < 2e-6
+
+
 def test_linear_quant_two_pass_scratch_entry_point():
     """dlp_linear's caller-provided-scratch contract still holds (used when DLP_GEMM_DEQUANT_SCRATCH=1)."""
     import ctypes as C
