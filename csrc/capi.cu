@@ -137,8 +137,9 @@ int dlp_rs_norm_ag(const dlp_rs_norm_ag_desc* d, void* stream) {
 int dlp_gemm_wait_expired(int* out) {
     DLP_REQUIRE(out, "dlp_gemm_wait_expired: null argument");
     *out = 0;
-    const int rc = gemm_pair_expired(out);
-    return rc ? rc : gemm_quant_small_expired(out);
+    int rc = gemm_pair_expired(out);
+    if (!rc) rc = gemm_quant_small_expired(out);
+    return rc ? rc : attn_prefill_expired(out);
 }
 
 static int linear_impl(const dlp_weight* w0, const dlp_weight* w1, const void* x, const float* norm_w, float eps, void* y,

@@ -402,6 +402,26 @@ def test_attn_prefill_causal(D, Hq, Hkv, T, pos0, page, impl):
     assert nmse(ref, out) < 5e-4
 
 
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 80, 8), (64, 72, 24), (64, 128, 128)])      # tiles of two heads; of 256 queries (3 and 1 heads to a key head)
+@pytest.mark.parametrize("T,pos0,page", [(257, 0, 64), (300, 129, 16), (384, 1000, 128), (520, 1, 32)])
+def test_attn_prefill_two_tiles(D, Hq, Hkv, T, pos0, page):
+    """Flash-prefill with two query tiles a block: last tiles of one row and a second tile that is not there, several key tiles, keys that end
+    inside a page, scores that grow by more than 2^8 on the way (the output is rescaled).  Against 64 bits; the weights and the output are fp16."""
+    n_need = (pos0 + T + page - 1) // page
+    kc, vc = _fill_cache(n_need + 3, Hkv, page, D, seed=1)
+    kc *= torch.linspace(0.2, 4, n_need + 3, device=DEV).view(-1, 1, 1, 1).to(kc.dtype)
+    row = torch.arange(n_need).to(torch.int32).to(DEV)
+    q = (torch.randn(T, Hq * D, device=DEV, generator=torch.Generator(DEV).manual_seed(4)) / math.sqrt(D)).half()
+    out = ops.attn_prefill(q, kc, vc, row, pos0, Hq, Hkv, D)
+    k, v = (c[row.long()].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :pos0 + T].double() for c in (kc, vc))
+    hidden = torch.arange(pos0 + T, device=DEV)[None] > pos0 + torch.arange(T, device=DEV)[:, None]
+    ref = torch.empty(T, Hq, D, dtype=torch.float64, device=DEV)
+    for h in range(Hq):
+        s = (q.view(T, Hq, D)[:, h].double() @ k[h * Hkv // Hq].T).masked_fill(hidden, -math.inf)
+        ref[:, h] = torch.softmax(s, -1) @ v[h * Hkv // Hq]
+    assert nmse(ref.view(T, -1), out) < 3e-7
+
+
 def test_argmax_and_sampler():
     R, V = 3, 32000
     lg = torch.randn(R, V, device=DEV)
