@@ -756,3 +756,22 @@ def test_gemm_split_k_workspace_fixup(t, T, mode):
         assert torch.equal(outs[0], outs[1])
     ws = ops.gemm_workspace(torch.device(DEV))
     assert int(ws[:16384].view(torch.int32).abs().sum()) == 0          # every tile counter went back to zero
+
+
+def test_rope_rows_of_a_prompt():
+    """RoPE of many tokens at once (one block a token) against the one-pair-a-thread kernel: whole and partial rotation, both pairings, negative slots."""
+    T, Hq, Hkv, page = 130, 6, 2, 16
+    for D, n_rot in ((64, 64), (128, 128), (128, 96), (64, 32)):
+        for neox in (False, True):
+            g = torch.Generator(DEV).manual_seed(D + n_rot)
+            qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, generator=g).half()
+            pos = torch.randint(0, 5000, (T,), device=DEV, generator=g).to(torch.int32)
+            slot = torch.randperm(T + 40, device=DEV, generator=g)[:T].to(torch.int32)
+            slot[::7] = -1
+            inv = (10000.0 ** (-torch.arange(0, n_rot // 2).double() * 2 / n_rot)).float().to(DEV)
+            got, want = ([torch.zeros(T, Hq * D, device=DEV, dtype=torch.float16)] + [torch.zeros(12, Hkv, page, D, device=DEV, dtype=torch.float16) for _ in range(2)] for _ in range(2))
+            ops.rope_kv(qkv, pos, slot, inv, got[1], got[2], Hq, Hkv, D, neox, q_out=got[0])
+            for i in range(0, T, 5):                    # (few tokens: the other kernel)
+                ops.rope_kv(qkv[i:i + 5], pos[i:i + 5], slot[i:i + 5], inv, want[1], want[2], Hq, Hkv, D, neox, q_out=want[0][i:i + 5])
+            for a, b in zip(got, want):
+                assert nmse(b, a) < 1e-8, (D, n_rot, neox)
