@@ -149,6 +149,9 @@ int gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, vo
 int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, int ldx, void* y, int ldy, int T, int epilogue,
                int split_k, cudaStream_t stream, const GemmCollective* coll = nullptr, const GemmGroup* grp = nullptr, void* ws = nullptr,
                size_t ws_bytes = 0);
+// the same for prompts: pieces of the weights unpacked to `scratch` (at least 256 rows of fp16, twice with w1), each multiplied by gemm_f16
+int gemm_quant_pieces(const QWeight& w0, const QWeight* w1, int wtype, const void* x, void* y, int ldy, int T, int epilogue, void* scratch,
+                      size_t scratch_bytes, cudaStream_t stream);
 // *out |= 1 when a bounded wait of the named kernels has run out on the current device since the library was loaded
 int gemm_pair_expired(int* out);
 int gemm_quant_small_expired(int* out);

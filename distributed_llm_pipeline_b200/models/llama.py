@@ -378,7 +378,7 @@ class LlamaEngine(EngineCore):
         ops.linear(lw.router_wp, xn, "f32", out=b["logits"][:T])     # router (padded to a full 128-row tile for the GEMM sizes)
         ops.moe_route_ex(b["logits"][:T], nE, k, cfg.moe_norm_topk, b["ids"][:A], b["w"][:A])
         per = max(1, A // nE)
-        bt = 16 if per <= 16 else 32 if per <= 32 else 64 if per <= 96 else 128
+        bt = 16 if per <= 16 else 32 if per <= 32 else 64 if per <= 96 or lw.e_gate_s.wtype.name.startswith("Q") else 128      # (block types: gemm_quant_small.cuh)
         ops.moe_plan(b["ids"][:A], nE, bt, b["plan"])
         ops.moe_gather(xn, b["plan"], k, A, b["xs"][:A])
         ops.linear_grouped(lw.e_gate_s, b["xs"][:A], b["act"][:A], "swiglu", nE, F, bt, b["plan"], w_up=lw.e_up_s)

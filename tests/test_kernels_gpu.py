@@ -160,7 +160,7 @@ def test_linear_quant_dequant_fused_gemm(t, T, N, K):
 
 
 @pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
-@pytest.mark.parametrize("T,N,K", [(5, 128, 256), (16, 200, 512), (17, 126, 768), (33, 384, 2304), (64, 130, 4096), (65, 256, 512)])
+@pytest.mark.parametrize("T,N,K", [(5, 128, 256), (16, 200, 512), (17, 126, 768), (33, 384, 2304), (64, 130, 4096), (65, 256, 512), (192, 384, 512)])
 def test_linear_quant_few_tokens(t, T, N, K):
     """Token tiles of 16, 32 and 64 (and the first size behind them), partial row tiles, one unit of columns up to several splits of K.  The weights
     enter as fp16 values (relative 2^-12 on average, squared 2e-8 with the margin of the few that round the other way); sums are fp32."""
@@ -172,6 +172,21 @@ def test_linear_quant_few_tokens(t, T, N, K):
     acc = torch.ones(T, N, device=DEV)
     assert nmse(ref + 1, ops.linear(w, x, "add", out=acc)) < 2e-7
     assert nmse(ref, ops.linear(w, x, "f16")) < 4e-7          # (and the rounding of the output)
+    assert nmse(torch.nn.functional.silu(ref) * (x.double() @ exact_u.double().T), ops.linear(w, x, "swiglu", w_up=u)) < 2e-6
+
+
+@pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
+@pytest.mark.parametrize("T,N,K,kib", [(193, 256, 256, 256), (300, 700, 512, 512), (1025, 1280, 768, 1 << 16)])
+def test_linear_quant_prompt_in_pieces(t, T, N, K, kib):
+    """Prompts on block types: one row tile a piece, pieces of which the last is partial, the whole matrix at once; bounds as for few tokens."""
+    w, exact = _w(N, K, t, 1)
+    u, exact_u = _w(N, K, t, 2)
+    x = torch.randn(T, K, device=DEV, generator=torch.Generator(DEV).manual_seed(3)).half()
+    ref = x.double() @ exact.double().T
+    scratch = torch.empty(kib << 10, dtype=torch.uint8, device=DEV)
+    assert nmse(ref, ops.linear(w, x, "f32", scratch=scratch)) < 2e-7 and nmse(ref, ops.linear(w, x, "f32")) < 2e-7
+    acc = torch.ones(T, N, device=DEV)
+    assert nmse(ref + 1, ops.linear(w, x, "add", out=acc, scratch=scratch)) < 2e-7
     assert nmse(torch.nn.functional.silu(ref) * (x.double() @ exact_u.double().T), ops.linear(w, x, "swiglu", w_up=u)) < 2e-6
 
 
