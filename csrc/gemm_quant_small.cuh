@@ -311,9 +311,9 @@ gemm_quant_small_kernel(const __grid_constant__ QsMaps tw0, const __grid_constan
             d0 = e0;
             d1 = e1;
         }
+        if (!grouped) pdl_wait();                               // the epilogue reads and writes what a predecessor may still use
         pdl_launch_dependents();
         if (group == 0) {
-            if (!grouped) pdl_wait();                           // the epilogue reads and writes what a predecessor may still use
             mbar_wait_b(done, 0);
             gemm_drain<BT, NA, 0>(p, tmem_base, done, true, n_out0, t0, t_end);
         }

@@ -316,6 +316,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     int t0 = blockIdx.y * BT;           // first token row (B operand, output row)
     int t_end = p.T;                    // output rows >= t_end are not stored
     const int n_out0 = n0;              // first output column
+    // Weights are static: in a plain launch the first stages of them are requested, and barriers and tensor memory set up, while the predecessor
+    // still runs.  Everything else waits for it: the tokens, what a collective or the table of a grouped launch says, and the epilogue.
+    const bool ahead = p.grp.tile_expert == nullptr && p.coll.x_flags == nullptr;
+    if (!ahead) pdl_wait();
     if (p.grp.tile_expert != nullptr) {
         // grouped launch: this token tile belongs to one expert; its weight rows sit at expert * rows_per_expert in the stack
         if ((int)blockIdx.y >= *p.grp.n_tiles) return;          // (uniform over the CTA, before any barrier / TMEM allocation)
@@ -366,17 +370,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                 }
                 fence_proxy_async_global();
             }
-            int stage = 0;
-            uint32_t phase = 0;
-            for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait(&empty_bar[stage], phase ^ 1);
-                mbar_expect_tx(&full_bar[stage], QUANT ? Cfg::B_BYTES : Cfg::STAGE_BYTES);
+            auto load_w = [&](int kb, int s) {
+                mbar_expect_tx(&full_bar[s], QUANT ? Cfg::B_BYTES : Cfg::STAGE_BYTES);
                 const int kc = (kb_begin + kb) * GEMM_BK;
                 if (!QUANT) {
-                    tma_load_2d(smem_a0 + stage * Cfg::A_BYTES, &tm_w0, &full_bar[stage], kc, n0);
-                    if (NA == 2) tma_load_2d(smem_a1 + stage * Cfg::A_BYTES, &tm_w1, &full_bar[stage], kc, n0);
+                    tma_load_2d(smem_a0 + s * Cfg::A_BYTES, &tm_w0, &full_bar[s], kc, n0);
+                    if (NA == 2) tma_load_2d(smem_a1 + s * Cfg::A_BYTES, &tm_w1, &full_bar[s], kc, n0);
                 }
-                tma_load_2d(smem_b + stage * Cfg::B_BYTES, &tm_x, &full_bar[stage], kc, t0);
+            };
+            const int first = min(STAGES, num_kb);
+            for (int kb = 0; kb < first; ++kb) load_w(kb, kb);
+            if (ahead) pdl_wait();
+            for (int kb = 0; kb < first; ++kb) tma_load_2d(smem_b + kb * Cfg::B_BYTES, &tm_x, &full_bar[kb], (kb_begin + kb) * GEMM_BK, t0);
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int kb = first; kb < num_kb; ++kb) {
+                mbar_wait(&empty_bar[stage], phase);
+                load_w(kb, stage);
+                tma_load_2d(smem_b + stage * Cfg::B_BYTES, &tm_x, &full_bar[stage], (kb_begin + kb) * GEMM_BK, t0);
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -423,6 +434,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
+        pdl_wait();
+        pdl_launch_dependents();
         gemm_drain<BT, NA, AB_FMT>(p, tmem_base, tmem_full_bar, num_kb > 0, n_out0, t0, t_end);
     }
     tc_fence_before();
@@ -459,8 +472,7 @@ static int launch_gemm(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUt
     if (first_use_on_device((const void*)kern))
         DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     dim3 grid((p.N + GEMM_BM - 1) / GEMM_BM, p.grp.tile_expert ? p.grp.max_tiles : (p.T + BT - 1) / BT, splits);
-    kern<<<grid, 192, Cfg::SMEM_BYTES, stream>>>(tw0, tw1, tx, p, qw0, qw1);
-    DLP_LAUNCH_CHECK();
+    DLP_CHECK_CUDA(launch_pdl(kern, grid, dim3(192), Cfg::SMEM_BYTES, stream, tw0, tw1, tx, p, qw0, qw1));
     return 0;
 }
 
