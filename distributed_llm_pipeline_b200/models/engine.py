@@ -240,7 +240,7 @@ class EngineCore:
         while len(seq.pages) > keep_pages:
             self.kv.free.append(seq.pages.pop())
         seq.length = new_len
-        self.seq_len_dev[sid] = new_len
+        self.seq_len_dev[sid:sid + 1].fill_(new_len)      # (a launch; an item assignment copies from the host)
 
     def copy_seq(self, src: int, dst: int, n: int | None = None):
         """Copy the first `n` cached tokens (default: all) of sequence `src` into `dst` (which is overwritten).
@@ -277,15 +277,6 @@ class EngineCore:
         self._sync_sampling(sids)
         rows = torch.tensor(sids, dtype=torch.int32, device=self.device)
         return ops.sample_dev(logits.contiguous(), self.samp, rows, torch.empty(len(sids), dtype=torch.int32, device=self.device)).tolist()
-
-    def _advance_inputs(self, sid: int, T: int):
-        """Grow the sequence's pages for T more tokens; positions and cache slots of those tokens (host int32)."""
-        seq = self.seqs[sid]
-        self.kv.ensure(seq, seq.length + T)
-        pos = torch.arange(seq.length, seq.length + T, dtype=torch.int32)
-        pages = torch.tensor(seq.pages, dtype=torch.int32)
-        slot = pages[(pos // self.page_size).long()] * self.page_size + pos % self.page_size
-        return pos, slot.to(torch.int32)
 
     # ---- decode -----------------------------------------------------------------------------------
     @torch.no_grad()

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from ..ops import api as ops
@@ -373,13 +374,20 @@ class LayeredEngine(EngineCore):
         return b
 
     def _mixed_batch(self, parts: list[tuple[int, list[int]]]) -> tuple[torch.Tensor, Batch]:
-        """Grow every sequence by its tokens (short parts first) and upload the description in one copy."""
+        """Grow every sequence by its tokens (short parts first) and upload the description in one copy.  (Lists and numpy: a torch call per
+        sequence and column costs more than the GPU takes for a small step.)"""
         lens = [len(t) for _, t in parts]
-        T = sum(lens)
-        pos, slot = zip(*(self._advance_inputs(sid, len(t)) for sid, t in parts))
-        cols: list[torch.Tensor] = [torch.cat([torch.as_tensor(t, dtype=torch.int32) for _, t in parts]), torch.cat(pos), torch.cat(slot),
-                                    torch.cat([torch.full((len(t),), sid, dtype=torch.int32) for sid, t in parts])]
-        ends = torch.tensor(lens).cumsum(0).tolist()
+        T, ps = sum(lens), self.page_size
+        places = []                                     # positions and cache slots of every part
+        for (sid, _), n in zip(parts, lens):
+            seq = self.seqs[sid]
+            self.kv.ensure(seq, seq.length + n)
+            first = seq.length // ps
+            pos = np.arange(seq.length, seq.length + n, dtype=np.int32)
+            places.append((pos, np.array(seq.pages[first:], dtype=np.int32)[pos // ps - first] * ps + pos % ps))
+        cols: list = [[x for _, t in parts for x in t], np.concatenate([p for p, _ in places]), np.concatenate([s for _, s in places]),
+                      np.repeat([sid for sid, _ in parts], lens)]
+        ends = np.cumsum(lens).tolist()
         segs = [(sid, hi - n, hi) for (sid, _), n, hi in zip(parts, lens, ends)]
         groups = [[g for g in segs if (g[2] - g[1] >= self.long_from) == is_long] for is_long in (False, True)]
         assert [g for grp in groups for g in grp] == segs
@@ -388,7 +396,7 @@ class LayeredEngine(EngineCore):
             lists = [[x for g in grp for x in g[1:]], [g[0] for g in grp]]
             for size in self._chunk_sizes if is_long else ():
                 lists += lops.scan_chunk_table([g[1:] for g in grp], size)
-            cols += [torch.tensor(x, dtype=torch.int32) for x in lists]
+            cols += lists
         shapes = []
         for kind in self._latent_kinds:
             H, _, Rc = kind
@@ -397,7 +405,7 @@ class LayeredEngine(EngineCore):
                     continue
                 bm = lops.latent_tile_rows(H, sum(lens[:n]), Rc)
                 row0, rows = self._tile_lists(H, lens[:n], bm)
-                cols += [torch.tensor(row0, dtype=torch.int32), torch.tensor(rows, dtype=torch.int32)]
+                cols += [row0, rows]
                 shapes.append(((kind, only_short), bm, len(row0)))
         for R in self._att_groups:
             for only_short in (False, True):
@@ -406,14 +414,15 @@ class LayeredEngine(EngineCore):
                     continue
                 bm, n = lops.gqa_tile(R, max(g[2] - g[1] for g in part))
                 row0, rows = self._token_tiles([g[1:] for g in part], n)
-                cols += [torch.tensor(row0, dtype=torch.int32), torch.tensor(rows, dtype=torch.int32)]
+                cols += [row0, rows]
                 shapes.append((("tokens", R, only_short), bm, len(row0)))
         if groups[1] and self._att_flash:       # the tiles with the longest context first
             order = sorted(((self.seqs[sid].length + t - lo, t, n) for sid, lo, hi in groups[1] for t, n in zip(*self._token_tiles([(lo, hi)], lops.FLASH_TILE))), reverse=True)
             row0, rows = [t for _, t, _ in order], [n for _, _, n in order]
-            cols += [torch.tensor(row0, dtype=torch.int32), torch.tensor(rows, dtype=torch.int32)]
+            cols += [row0, rows]
             shapes.append(("flash", lops.FLASH_TILE, len(row0)))
-        dev = iter(torch.cat(cols).to(self.device).split([c.numel() for c in cols]))
+        host = [np.asarray(c, dtype=np.int32) for c in cols]
+        dev = iter(torch.from_numpy(np.concatenate(host)).to(self.device).split([c.size for c in host]))
         ids, pos_d, slot_d, tok_slot = (next(dev) for _ in range(4))
         most = [max((hi - lo for _, lo, hi in grp), default=0) for grp in groups]
         short = Segments(len(groups[0]), next(dev), next(dev), longest=most[0])
@@ -430,8 +439,8 @@ class LayeredEngine(EngineCore):
         pending = self._forward(ids, b)
         for sid, t in parts:
             self.seqs[sid].length += len(t)
-        lens = torch.tensor([[sid, self.seqs[sid].length] for sid, _ in parts], dtype=torch.int32).to(self.device)
-        self.seq_len_dev[lens[:, 0].long()] = lens[:, 1]
+        lens = torch.tensor([[sid, self.seqs[sid].length] for sid, _ in parts]).to(self.device)
+        self.seq_len_dev.index_copy_(0, lens[:, 0], lens[:, 1].int())
         return pending
 
     # ---- public ---------------------------------------------------------------------------------------------
@@ -480,8 +489,12 @@ class LayeredEngine(EngineCore):
                 h = self._settle(sum(len(t) for _, t in parts), pending)
                 for k in range(0, len(rows), self.max_rows):
                     idx = torch.tensor(rows[k:k + self.max_rows], dtype=torch.long, device=self.device)
+                    to = dst[k:k + self.max_rows]
+                    if to == list(range(len(to))):          # the first rows of the result, in order: straight into it
+                        self._head_rows(Rows(h[idx], self.E), len(idx), out[:len(to)])
+                        continue
                     lg = self._head_rows(Rows(h[idx], self.E), len(idx), torch.empty(len(idx), self.cfg.vocab_size, dtype=torch.float32, device=self.device))
-                    out[torch.tensor(dst[k:k + self.max_rows], dtype=torch.long, device=self.device)] = lg
+                    out[torch.tensor(to, dtype=torch.long, device=self.device)] = lg
         if self.device.type == "cuda":
             lops.check_waits()
         return out
