@@ -35,8 +35,6 @@ class PagedKVCache:
         self.free = list(range(n_pages - 1, -1, -1))
         self.block_table = torch.zeros(max_seqs, max_pages_per_seq, dtype=torch.int32, device=device)
         self.block_table_host = torch.zeros(max_seqs, max_pages_per_seq, dtype=torch.int32)
-        if torch.device(device).type == "cuda":
-            self.block_table_host = self.block_table_host.pin_memory()
 
     @property
     def k(self):
@@ -66,6 +64,8 @@ class PagedKVCache:
             seq.pages.append(pg)
             grew = True
         if grew:
+            # from pageable memory: the row is taken before this returns (a pinned one would be read when the stream gets there, with what the
+            # sequence, or the next one in its slot, has written to it by then)
             self.block_table[seq.sid].copy_(self.block_table_host[seq.sid], non_blocking=True)
 
     def release(self, seq: Sequence):
@@ -194,8 +194,11 @@ class EngineCore:
             raise RuntimeError("no free sequence slots")
         sid = self._free_sids.pop()
         self.seqs[sid] = Sequence(sid)
-        self.seq_len_dev[sid] = 0        # a decode step may be the sequence's first: the device-side length starts over with the slot
+        self._set_len(sid, 0)            # a decode step may be the sequence's first: the device-side length starts over with the slot
         return sid
+
+    def _set_len(self, sid: int, n: int):
+        self.seq_len_dev[sid:sid + 1].fill_(n)      # (a launch in the stream; an item assignment copies from the host and waits for the stream)
 
     def free_seq(self, sid: int):
         self.kv.release(self.seqs.pop(sid))
@@ -240,7 +243,7 @@ class EngineCore:
         while len(seq.pages) > keep_pages:
             self.kv.free.append(seq.pages.pop())
         seq.length = new_len
-        self.seq_len_dev[sid:sid + 1].fill_(new_len)      # (a launch; an item assignment copies from the host)
+        self._set_len(sid, new_len)
 
     def copy_seq(self, src: int, dst: int, n: int | None = None):
         """Copy the first `n` cached tokens (default: all) of sequence `src` into `dst` (which is overwritten).
@@ -260,7 +263,7 @@ class EngineCore:
         if self.rstate and n:
             self.rstate.copy(src, dst)
         d.length = n
-        self.seq_len_dev[dst] = n
+        self._set_len(dst, n)
 
     @property
     def can_rollback(self) -> bool:

@@ -630,7 +630,7 @@ class LlamaEngine(EngineCore):
             seq.length = pos0 + T
             if not self.last_stage:
                 outs.append(self.h[:T].clone())
-        self.seq_len_dev[sid] = seq.length
+        self._set_len(sid, seq.length)
         if not self.last_stage:
             return torch.cat(outs, 0)
         if sp:

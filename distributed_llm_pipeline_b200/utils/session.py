@@ -84,5 +84,5 @@ def load_sequence(eng, sid: int, path: str) -> dict:
         for _, _, st in eng.rstate.each():
             st[sid] = payload(st[sid].numel() * 4).view(torch.float32).view(st.shape[1:]).to(eng.device)
         seq.length = n
-        eng.seq_len_dev[sid] = n
+        eng._set_len(sid, n)
     return hdr

@@ -180,3 +180,22 @@ def test_moe_engine_any_token_count_on_device(tmp_models, key, T):
         lg = eng.decode([sid], [t], sample=False)[0]
         assert nmse(ref_logits[i + 1], lg) < 1e-3, i
     assert any(k[:2] == (1, False) for k in eng._graphs)
+
+
+def test_block_table_row_is_taken_when_it_is_copied(tmp_models):
+    """A prompt that is still queued keeps its pages when its slot goes to another sequence meanwhile: nothing waits for the stream between the two."""
+    eng = LlamaEngine(load_weights(tmp_models[("tiny", "F16")], "cuda"), n_ctx=256, max_seqs=2, page_size=16, max_batch_tokens=64)
+    table = eng.kv.block_table
+    sid = eng.alloc_seq()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)                  # the stream is busy for some 10 ms
+    eng.kv.ensure(eng.seqs[sid], 48)
+    first, seen = list(eng.seqs[sid].pages), table[sid].clone()
+    eng.free_seq(sid)
+    other = [eng.kv.free.pop() for _ in range(3)]  # (the same slot, other pages)
+    again = eng.alloc_seq()
+    assert again == sid
+    eng.kv.ensure(eng.seqs[again], 48)
+    assert eng.seqs[again].pages != first
+    eng.kv.free.extend(other)
+    assert seen[:3].tolist() == first and table[sid][:3].tolist() == eng.seqs[again].pages
