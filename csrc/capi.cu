@@ -139,6 +139,7 @@ int dlp_gemm_wait_expired(int* out) {
     *out = 0;
     int rc = gemm_pair_expired(out);
     if (!rc) rc = gemm_quant_small_expired(out);
+    if (!rc) rc = gemv_expired(out);
     return rc ? rc : attn_prefill_expired(out);
 }
 

@@ -11,6 +11,7 @@
 
 #include "kernels.cuh"
 #include "tpcomm.cuh"
+#include "waits.cuh"
 
 namespace dlp {
 
@@ -431,10 +432,22 @@ static int resident_cluster_blocks(Kern kern, unsigned cl, size_t smem, int thre
     return want < cap ? want : cap;
 }
 
+// How much of an SM's 256 KB is shared memory is left to the driver otherwise, and it keeps what the largest neighbour in the stream asked for:
+// behind attention (196 KB for two blocks) the loads in flight of these kernels - 128 KB of registers to fill an SM - found 28 KB of L1 to return
+// through, and 8 layers of Llama-8B decoded in Q8_0 at 815 us a token instead of 635 (all for shared memory: 1,220; a third: 704).  So half of it is
+// shared memory for one and two tokens, room for two blocks of the widest rows (2 x 52 KB).  Four tokens need more of it and are bound by
+// arithmetic: left to the driver, 1,310 us a step in Q4_K_M against 1,430.
+template <typename Kern>
+static int gemv_first_use(Kern kern, int T) {
+    if (!first_use_on_device((const void*)kern)) return 0;
+    DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    if (T <= 2) DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 50));
+    return 0;
+}
+
 template <typename Kern>
 static int launch_gemv_v3(Kern kern, const GemvParams& p, int U, size_t x_smem, cudaStream_t stream) {
-    if (first_use_on_device((const void*)kern))
-        DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    if (int rc = gemv_first_use(kern, p.T)) return rc;
     const bool dual = p.out_mode == GV_SWIGLU_F16;
     const int rpu = dual ? 1 : 2;
     const int groups = (p.w0.N + rpu - 1) / rpu;
@@ -774,14 +787,18 @@ __device__ __forceinline__ int dp4a4(const uint32_t (&q)[4], const uint4& x) {
     return __dp4a((int)q[3], (int)x.w, s);
 }
 
+__device__ __forceinline__ __half2 u32_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 __device__ __forceinline__ float us2f(unsigned short h) { return __half2float(__ushort_as_half(h)); }
 
-// dot of one raw chunk with token t's int8 activations; xq int8 [K], xd fp32 [K/32] scales, xs16 fp32 [K/16] exact sums,
-// xqs16 int [K/16] sums of the int8 values.  `c` is the chunk index (needed to pick the sub-block scales).  Unsigned quant
+// dot of one raw chunk with token t's int8 activations; xq int8 [K], xd fp32 [K/32] scales, xqs16 int [K/16] sums of the int8 values.  `c` is the chunk index (needed to pick the sub-block scales).  Unsigned quant
 // values are centred ( sum (q-z) xq = dp4a(q, xq) - z * sum xq ), which keeps the activation-rounding noise off the large offset
 // term; the sum of xq per 16 values comes from the prologue instead of a second set of dp4a per chunk.
+// The 4- and 5-bit types take, with S = sum of x, s = sum of xq and D = scale of 32 values, {D, z (S - D s), S} in one load (xb):
+//   sum_i (scale q_i - min) x_i  ~=  scale (D dot_int(q, xq) + z (S - D s)) - min S
+// (Ten loads of the sums by themselves and the scales of one sub-block at a time: Q4_K gate and up of Llama-8B 23.4 us instead of 20.0, 4 tokens 56
+// instead of 40; 128256 x 4096 91 instead of 77, 4 tokens 214 instead of 141.)
 template <int WT>
-__device__ __forceinline__ float qraw_dot(const QRaw<WT>& r, const int8_t* xq, const float* xd, const float* xs16, const int* xqs16,
+__device__ __forceinline__ float qraw_dot(const QRaw<WT>& r, const int8_t* xq, const float* xd, const int* xqs16, const float4* xb,
                                           int c, int k0, int k1) {
     if constexpr (WT == W_Q8_0) {
         const int rot = (c >> 1) & 3;                      // granule rotation of this 64-byte group (see the quantise prologue)
@@ -800,10 +817,12 @@ __device__ __forceinline__ float qraw_dot(const QRaw<WT>& r, const int8_t* xq, c
         const uint4 xa0 = *reinterpret_cast<const uint4*>(xg + ((rot & 3) << 4)), xa1 = *reinterpret_cast<const uint4*>(xg + (((1 + rot) & 3) << 4));
         const uint4 xb0 = *reinterpret_cast<const uint4*>(xg + (((2 + rot) & 3) << 4)), xb1 = *reinterpret_cast<const uint4*>(xg + (((3 + rot) & 3) << 4));
         const float2 dm = h2_to_f2(r.hdr.x);
-        int sc0, mn0, sc1, mn1;
-        scale_min_k4(r.hdr.y, r.hdr.z, r.hdr.w, 2 * j, sc0, mn0);
-        scale_min_k4(r.hdr.y, r.hdr.z, r.hdr.w, 2 * j + 1, sc1, mn1);
-        const float s0 = dm.x * sc0, s1 = dm.x * sc1;
+        // the 6-bit scales and mins of four sub-blocks at a time (the packing of scale_min_k4), then the two of this chunk
+        const uint32_t sc4 = j < 2 ? r.hdr.y & 0x3F3F3F3Fu : (r.hdr.w & 0x0F0F0F0Fu) | ((r.hdr.y >> 2) & 0x30303030u);
+        const uint32_t mn4 = j < 2 ? r.hdr.z & 0x3F3F3F3Fu : ((r.hdr.w >> 4) & 0x0F0F0F0Fu) | ((r.hdr.z >> 2) & 0x30303030u);
+        const uint32_t sc = sc4 >> (16 * (j & 1)), mn = mn4 >> (16 * (j & 1));
+        const float2 scf = __half22float2(__hsub2(u32_h2(__byte_perm(sc, 0x64646464u, 0x4140)), __float2half2_rn(1024.f)));
+        const float2 mnf = __half22float2(__hsub2(u32_h2(__byte_perm(mn, 0x64646464u, 0x4140)), __float2half2_rn(1024.f)));
         const uint32_t w0[4] = {r.qs0.x, r.qs0.y, r.qs0.z, r.qs0.w}, w1[4] = {r.qs1.x, r.qs1.y, r.qs1.z, r.qs1.w};
         uint32_t lo0[4], hi0[4], lo1[4], hi1[4];
 #pragma unroll
@@ -813,7 +832,6 @@ __device__ __forceinline__ float qraw_dot(const QRaw<WT>& r, const int8_t* xq, c
             lo1[i] = w1[i] & 0x0F0F0F0Fu;
             hi1[i] = (w1[i] >> 4) & 0x0F0F0F0Fu;
         }
-        constexpr int Z = (WT == W_Q5_K) ? 16 : 8;
         if constexpr (WT == W_Q5_K) {
             const uint32_t h0[4] = {r.qh0.x, r.qh0.y, r.qh0.z, r.qh0.w}, h1[4] = {r.qh1.x, r.qh1.y, r.qh1.z, r.qh1.w};
 #pragma unroll
@@ -824,11 +842,10 @@ __device__ __forceinline__ float qraw_dot(const QRaw<WT>& r, const int8_t* xq, c
                 hi1[i] |= ((h1[i] >> (2 * j + 1)) & 0x01010101u) << 4;
             }
         }
-        const int ka = k0 >> 4, kb = k1 >> 4;
-        const int ia = dp4a4(lo0, xa0) + dp4a4(lo1, xa1) - Z * (xqs16[ka] + xqs16[ka + 1]);
-        const int ib = dp4a4(hi0, xb0) + dp4a4(hi1, xb1) - Z * (xqs16[kb] + xqs16[kb + 1]);
-        const float b0 = (float)Z * s0 - dm.y * mn0, b1 = (float)Z * s1 - dm.y * mn1;
-        return s0 * xd[k0 >> 5] * (float)ia + s1 * xd[k1 >> 5] * (float)ib + b0 * (xs16[ka] + xs16[ka + 1]) + b1 * (xs16[kb] + xs16[kb + 1]);
+        const int ia = dp4a4(lo0, xa0) + dp4a4(lo1, xa1), ib = dp4a4(hi0, xb0) + dp4a4(hi1, xb1);
+        const float4 ta = xb[k0 >> 5], tb = xb[k1 >> 5];
+        const float pos = fmaf(scf.x, fmaf(ta.x, (float)ia, ta.y), scf.y * fmaf(tb.x, (float)ib, tb.y)), neg = fmaf(mnf.x, ta.z, mnf.y * tb.z);
+        return fmaf(dm.x, pos, -dm.y * neg);
     } else {   // Q6_K: stored value = q + 32
         const uint4 xa = *reinterpret_cast<const uint4*>(xq + k0);
         const uint4 xb = *reinterpret_cast<const uint4*>(xq + k1);
@@ -858,18 +875,17 @@ __global__ void __launch_bounds__(256, 2) gemv_quant_v3_kernel(const GemvParams 
     const unsigned kc_inv = (unsigned)((0x100000000ull + (unsigned)KC - 1) / (unsigned)KC);   // exact for u < 2^32 / KC (KC == 1 is special-cased: the reciprocal would not fit)
     const bool dual = p.out_mode == GV_SWIGLU_F16;
     const int rpu = dual ? 1 : 2;
-    // shared memory: fp16 x [NT][K] (stage_x output, AR staging behind it) | int8 xq [NT][K] | xd [NT][K/32] | xs16 [NT][K/16] | xqs16 [NT][K/16] | partials
+    // shared memory: fp16 x [NT][K] (stage_x output, AR staging behind it) | int8 xq [NT][K] | xd [NT][K/32], xqs16 [NT][K/16] or xb [NT][K/32] | partials
+    constexpr bool MINS = WT == W_Q4_K || WT == W_Q5_K;
     __half* xs = reinterpret_cast<__half*>(gv_smem);
     size_t off = (size_t)NT * K * 2 + ar_stage_bytes(p.ar_in.buf != nullptr, NT, K);
     off = (off + 15) & ~size_t(15);
     int8_t* xq = reinterpret_cast<int8_t*>(gv_smem + off);
     off += (size_t)NT * K;
+    float4* xb = reinterpret_cast<float4*>(gv_smem + off);
     float* xd = reinterpret_cast<float*>(gv_smem + off);
-    off += (size_t)NT * nb32 * 4;
-    float* xs16 = reinterpret_cast<float*>(gv_smem + off);
-    off += (size_t)NT * (K >> 4) * 4;
-    int* xqs16 = reinterpret_cast<int*>(gv_smem + off);
-    off += (size_t)NT * (K >> 4) * 4;
+    int* xqs16 = reinterpret_cast<int*>(xd + (size_t)NT * nb32);
+    off += MINS ? (size_t)NT * nb32 * 16 : (size_t)NT * (nb32 + (K >> 4)) * 4;
     float* partial = reinterpret_cast<float*>(gv_smem + off);
     __shared__ float red[32];
     __shared__ int next_unit;
@@ -903,8 +919,8 @@ __global__ void __launch_bounds__(256, 2) gemv_quant_v3_kernel(const GemvParams 
             chunk_offsets<WT>(c, k0, k1);
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                acc[0][t] = qraw_dot<WT>(buf[b][0], xq + (size_t)t * K, xd + (size_t)t * nb32, xs16 + (size_t)t * (K >> 4), xqs16 + (size_t)t * (K >> 4), c, k0, k1);
-                acc[1][t] = qraw_dot<WT>(buf[b][1], xq + (size_t)t * K, xd + (size_t)t * nb32, xs16 + (size_t)t * (K >> 4), xqs16 + (size_t)t * (K >> 4), c, k0, k1);
+                acc[0][t] = qraw_dot<WT>(buf[b][0], xq + (size_t)t * K, xd + (size_t)t * nb32, xqs16 + (size_t)t * (K >> 4), xb + (size_t)t * nb32, c, k0, k1);
+                acc[1][t] = qraw_dot<WT>(buf[b][1], xq + (size_t)t * K, xd + (size_t)t * nb32, xqs16 + (size_t)t * (K >> 4), xb + (size_t)t * nb32, c, k0, k1);
             }
         }
         float* dst = partial + ((size_t)g * KC + cu) * 2 * NT;
@@ -960,8 +976,15 @@ __global__ void __launch_bounds__(256, 2) gemv_quant_v3_kernel(const GemvParams 
         int qs4 = q0 + q1 + q2 + q3;
         qs4 += __shfl_xor_sync(0xffffffffu, qs4, 1);
         qs4 += __shfl_xor_sync(0xffffffffu, qs4, 2);         // integer sum over the same 16 values
-        if ((i & 7) == 0) xd[i >> 3] = d;
-        if ((i & 3) == 0) { xs16[i >> 2] = s4; xqs16[i >> 2] = qs4; }
+        if constexpr (MINS) {
+            constexpr float Z = WT == W_Q5_K ? 16.f : 8.f;
+            s4 += __shfl_xor_sync(0xffffffffu, s4, 4);
+            qs4 += __shfl_xor_sync(0xffffffffu, qs4, 4);
+            if ((i & 7) == 0) xb[i >> 3] = make_float4(d, Z * fmaf(-d, (float)qs4, s4), s4, 0.f);
+        } else {
+            if ((i & 7) == 0) xd[i >> 3] = d;
+            if ((i & 3) == 0) xqs16[i >> 2] = qs4;
+        }
     }
     __syncthreads();
 
@@ -1019,9 +1042,8 @@ __global__ void __launch_bounds__(256, 2) gemv_quant_v3_kernel(const GemvParams 
 }
 
 template <typename Kern>
-static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaStream_t stream, int chunk_w = 32) {
-    if (first_use_on_device((const void*)kern))
-        DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaStream_t stream, int chunk_w, bool mins) {
+    if (int rc = gemv_first_use(kern, p.T)) return rc;
     const bool dual = p.out_mode == GV_SWIGLU_F16;
     const int rpu = dual ? 1 : 2;
     const int groups = (p.w0.N + rpu - 1) / rpu;
@@ -1029,7 +1051,9 @@ static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaSt
     if (blocks > groups) blocks = groups;
     const unsigned cl = ar_cluster(p, blocks);
     const int K = p.w0.K, KC = ((K / chunk_w) + 31) >> 5;
-    const size_t fixed = ((x_smem + 15) & ~size_t(15)) + (size_t)p.T * (K + (K >> 5) * 4 + (K >> 4) * 8);
+    // (without mins: what the kernel uses and as much again of the sums that it no longer keeps - 2 tokens of 14,336 columns stay with the kernel
+    // below, 25 us against 37 for 4096 x 14336 in Q8_0)
+    const size_t fixed = ((x_smem + 15) & ~size_t(15)) + (size_t)p.T * (K + (K >> 5) * (mins ? 16 : 20));
     blocks = resident_cluster_blocks(kern, cl, fixed + 4096, 256, blocks);
     blocks -= blocks % (int)cl;
     const int max_groups = (groups + blocks - 1) / blocks + 1;
@@ -1038,6 +1062,196 @@ static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaSt
     DLP_CHECK_CUDA(launch_pdl_cluster(kern, dim3(blocks), dim3(256), smem, stream, cl, p));
     return 0;
 }
+
+// ---- Q6_K x one token through a ring in shared memory ------------------------------------------------------------------------------
+// Bound by the weights' bytes.  A lane's chunk of Q6_K is five loads, of which gemv_quant_v3_kernel holds three units in registers (spilled at
+// that): 43 % of the memory's rate.  Here one warp copies whole rows (contiguous in every plane) into a ring with cp.async.bulk, 90 KB a block, two
+// blocks an SM, the first stages before the predecessor has finished; the other eight take the rows of a stage (8 / R warps a row) from
+// shared memory, with the arithmetic of v3, and one warp sum per row.  Llama-8B shapes in us, before and now: 128256 x 4096 153 -> 90 (bytes: 66),
+// gate and up 38 -> 27, 4096 x 14336 22 -> 18, 6144 x 4096 10.9 -> 9.6.  (The other types gain nothing: 2 to 4 KB less a row to hold, and the way
+// through shared memory costs what it saves - Q8_0 gate and up 24 -> 30, Q4_K 23 -> 24.  Nor do 2 and 4 tokens: 4096 x 14336 25 -> 28.)
+struct RingCfg { int R, S, wpr; };       // rows of a stage (of each matrix), stages, warps of a row
+__host__ __device__ constexpr int ring_row_bytes(int K, int plane) { return plane == 0 ? K / 2 : plane == 1 ? K / 4 : K / 16; }      // low nibbles | high bits | scales
+
+__global__ void __launch_bounds__(288, 2) gemv_q6_ring_kernel(const GemvParams p, const RingCfg cfg) {
+    extern __shared__ __align__(16) uint8_t gv_smem[];
+    __shared__ uint64_t full[8], empty[8];
+    __shared__ float red[32];
+    const int K = p.w0.K, N = p.w0.N, R = cfg.R, S = cfg.S, wpr = cfg.wpr;
+    const bool dual = p.out_mode == GV_SWIGLU_F16;
+    const int nmat = dual ? 2 : 1, row_total = ring_row_bytes(K, 0) + ring_row_bytes(K, 1) + ring_row_bytes(K, 2), stage_bytes = R * row_total * nmat;
+    const int r_lo = (int)(((long long)N * blockIdx.x) / gridDim.x), r_hi = (int)(((long long)N * (blockIdx.x + 1)) / gridDim.x), rows = r_hi - r_lo;
+    const int n_st = (rows + R - 1) / R;
+    // ring | xq [K] | xd [K/32] | xqs16 [K/16] | partial sums [rows][wpr][nmat] | fp16 scales [nmat][rows][K/256]
+    int8_t* xq = reinterpret_cast<int8_t*>(gv_smem + (size_t)S * stage_bytes);
+    float* xd = reinterpret_cast<float*>(xq + K);
+    int* xqs16 = reinterpret_cast<int*>(xd + (K >> 5));
+    float* partial = reinterpret_cast<float*>(xqs16 + (K >> 4));
+    __half* d6 = reinterpret_cast<__half*>(partial + (size_t)rows * wpr * nmat);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool dyn_rows = p.row_off_dev != nullptr;
+    size_t roff = 0;                             // expert row offset (MoE), known only after the router kernel has finished
+    auto issue = [&](int it) {                   // one lane: request stage `it`
+        const int s = it % S, row0 = r_lo + it * R, n = min(R, r_hi - row0);
+        mbar_expect_tx(&full[s], (uint32_t)(n * row_total * nmat));
+        uint8_t* dst = gv_smem + (size_t)s * stage_bytes;
+        for (int m = 0; m < nmat; ++m) {
+            const QWeight& w = m ? p.w1 : p.w0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int rb = ring_row_bytes(K, i);
+                bulk_g2s(dst, (i == 0 ? w.base : i == 1 ? w.aux0 : w.aux1) + (roff + row0) * rb, (uint32_t)(n * rb), &full[s]);
+                dst += (size_t)R * rb;
+            }
+        }
+    };
+    auto scales = [&]() {
+        const int per = K >> 8;
+        for (int m = 0; m < nmat; ++m) {
+            const __half* src = reinterpret_cast<const __half*>((m ? p.w1 : p.w0).aux2) + (roff + r_lo) * per;
+            for (int i = tid; i < rows * per; i += 288) d6[m * rows * per + i] = src[i];
+        }
+    };
+    if (tid == 256) {
+        for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 8); }
+        mbar_fence_init();
+        if (!dyn_rows)
+            for (int it = 0; it < min(S, n_st); ++it) issue(it);      // weights are static: requested before the predecessor has finished
+    }
+    if (!dyn_rows) scales();
+    pdl_wait();
+    if (p.pdl_early) pdl_launch_dependents();
+    if (dyn_rows) {
+        roff = (size_t)(*p.row_off_dev) * p.row_off_mul;
+        if (tid == 256)
+            for (int it = 0; it < min(S, n_st); ++it) issue(it);
+        scales();
+    }
+    const float oscale = p.out_scale_dev ? *p.out_scale_dev : 1.f;
+    // quantise the activations: 4 values a thread, one scale per 32 (8 threads), straight from global memory
+    float rs = 0.f;
+    const float* h = reinterpret_cast<const float*>(p.x);
+    if (p.norm_w != nullptr) {
+        float ss = 0.f;
+        for (int k = tid * 4; k < K; k += 288 * 4) {
+            const float4 v = *reinterpret_cast<const float4*>(h + k);
+            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+        rs = rsqrtf(block_sum(ss, red) / (float)K + p.eps);
+    }
+    for (int i = tid; i < (K >> 2); i += 288) {
+        uint2 hv;
+        if (p.norm_w != nullptr) {
+            const float4 v = *reinterpret_cast<const float4*>(h + i * 4), g = *reinterpret_cast<const float4*>(p.norm_w + i * 4);
+            const __half2 u = __floats2half2_rn(v.x * rs * g.x, v.y * rs * g.y), w = __floats2half2_rn(v.z * rs * g.z, v.w * rs * g.w);
+            hv = make_uint2(*reinterpret_cast<const uint32_t*>(&u), *reinterpret_cast<const uint32_t*>(&w));
+        } else {
+            hv = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(p.x) + i * 4);
+        }
+        const float2 a = h2_to_f2(hv.x), b = h2_to_f2(hv.y);
+        float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y)));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+        const float d = amax / 127.f, inv = amax > 0.f ? 127.f / amax : 0.f;
+        const int q0 = __float2int_rn(a.x * inv), q1 = __float2int_rn(a.y * inv), q2 = __float2int_rn(b.x * inv), q3 = __float2int_rn(b.y * inv);
+        reinterpret_cast<uint32_t*>(xq)[i] = (uint32_t)(q0 & 0xff) | ((uint32_t)(q1 & 0xff) << 8) | ((uint32_t)(q2 & 0xff) << 16) | ((uint32_t)(q3 & 0xff) << 24);
+        int qs4 = q0 + q1 + q2 + q3;
+        qs4 += __shfl_xor_sync(0xffffffffu, qs4, 1);
+        qs4 += __shfl_xor_sync(0xffffffffu, qs4, 2);             // integer sum over 16 values
+        if ((i & 7) == 0) xd[i >> 3] = d;
+        if ((i & 3) == 0) xqs16[i >> 2] = qs4;
+    }
+    __syncthreads();                             // (barrier inits are visible as well)
+
+    if (warp == 8) {
+        if (elect_one())
+            for (int it = S; it < n_st; ++it) {
+                mbar_wait_b(&empty[it % S], ((it / S) - 1) & 1);
+                issue(it);
+            }
+        __syncwarp();
+    } else {
+        const int r = warp / wpr, sub = warp - r * wpr, nch = K / 32;
+        for (int it = 0; it < n_st; ++it) {
+            const int s = it % S, rl = it * R + r;
+            mbar_wait_b(&full[s], (it / S) & 1);
+            for (int m = 0; m < nmat && rl < rows; ++m) {
+                const uint8_t* ql = gv_smem + (size_t)s * stage_bytes + (size_t)m * R * row_total;
+                const uint8_t* qh = ql + (size_t)R * ring_row_bytes(K, 0) + (size_t)r * ring_row_bytes(K, 1);
+                const signed char* sc = reinterpret_cast<const signed char*>(ql) + (size_t)R * (ring_row_bytes(K, 0) + ring_row_bytes(K, 1)) + (size_t)r * ring_row_bytes(K, 2);
+                ql += (size_t)r * ring_row_bytes(K, 0);
+                const __half* dr = d6 + (size_t)(m * rows + rl) * (K >> 8);
+                float acc = 0.f;
+#pragma unroll 2
+                for (int c = sub * 32 + lane; c < nch; c += 32 * wpr) {
+                    const int blk = c >> 3, cc = c & 7, half = cc >> 2, l0 = (cc & 3) * 16, lq = l0 & 31, upper = l0 >> 5;
+                    QRaw<W_Q6_K> w;
+                    w.ql = *reinterpret_cast<const uint4*>(ql + blk * 128 + half * 64 + l0);
+                    w.qh = *reinterpret_cast<const uint4*>(qh + blk * 64 + half * 32 + lq);
+                    const signed char* s0 = sc + blk * 16 + half * 8 + (lq >> 4) + upper * 2;
+                    w.s0 = s0[0];
+                    w.s1 = s0[4];
+                    w.d = __half_as_ushort(dr[blk]);
+                    int k0, k1;
+                    chunk_offsets<W_Q6_K>(c, k0, k1);
+                    acc += qraw_dot<W_Q6_K>(w, xq, xd, xqs16, nullptr, c, k0, k1);
+                }
+                acc = warp_sum(acc);
+                if (lane == 0) partial[(size_t)(rl * wpr + sub) * nmat + m] = acc;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
+        }
+    }
+    pdl_launch_dependents();
+    gemm_wait_aftermath();
+    __syncthreads();
+    for (int rl = tid; rl < rows; rl += 288) {
+        float v0 = 0.f, v1 = 0.f;
+        for (int u = 0; u < wpr; ++u) {
+            v0 += partial[(size_t)(rl * wpr + u) * nmat];
+            if (dual) v1 += partial[(size_t)(rl * wpr + u) * nmat + 1];
+        }
+        if (!dual) v0 *= oscale;
+        const int row = r_lo + rl;
+        if (p.out_mode == GV_STORE_F16) reinterpret_cast<__half*>(p.y)[row] = __float2half_rn(v0);
+        else if (p.out_mode == GV_STORE_F32) reinterpret_cast<float*>(p.y)[row] = v0;
+        else if (p.out_mode == GV_ADD_F32) reinterpret_cast<float*>(p.y)[row] += v0;
+        else reinterpret_cast<__half*>(p.y)[row] = __float2half_rn(gv_silu(v0) * v1);
+    }
+}
+
+// -2: the caller takes another kernel (an all-reduce is folded in or pushed out, planes that cp.async.bulk cannot read, no room)
+static int launch_gemv_q6_ring(const GemvParams& p, cudaStream_t stream) {
+    if (p.T != 1 || p.ar_in.buf != nullptr || p.out_mode == GV_PUSH_F32) return -2;
+    const int K = p.w0.K, N = p.w0.N, nmat = p.out_mode == GV_SWIGLU_F16 ? 2 : 1;
+    auto off = [](const void* q) { return reinterpret_cast<uintptr_t>(q) & 15; };
+    for (int m = 0; m < nmat; ++m) {
+        const QWeight& w = m ? p.w1 : p.w0;
+        if (off(w.base) || off(w.aux0) || off(w.aux1)) return -2;
+    }
+    if (off(p.x) || off(p.norm_w)) return -2;
+    auto kern = gemv_q6_ring_kernel;
+    const int blocks = sm_count() * 2 < N ? sm_count() * 2 : N, rows = (N + blocks - 1) / blocks;
+    for (int R = 8; R >= 1; R >>= 1) {
+        const int wpr = 8 / R, need = (rows + R - 1) / R;
+        const size_t stage = (size_t)R * (K / 2 + K / 4 + K / 16) * nmat, budget = 112 * 1024;
+        const size_t fixed = (size_t)K + (K >> 5) * 4 + (K >> 4) * 4 + (size_t)rows * wpr * nmat * 4 + (size_t)nmat * rows * (K >> 8) * 2;
+        if (fixed >= budget) continue;
+        int S = (int)((budget - fixed) / stage);
+        if (S > 8) S = 8;
+        if (S > need) S = need;
+        if (S < 1 || (S < 3 && S < need)) continue;         // (a shallower ring leaves gaps: fewer rows a stage)
+        if (first_use_on_device((const void*)kern)) DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+        const RingCfg cfg = {R, S, wpr};
+        DLP_CHECK_CUDA(launch_pdl(kern, dim3(blocks), dim3(288), (size_t)S * stage + fixed, stream, p, cfg));
+        return 0;
+    }
+    return -2;
+}
+
+int gemv_expired(int* out) { return gemm_wait_flag(out); }
 
 // ---- MoE router: softmax over all experts -> top-k -> renormalise (llama-graph.cpp:1039-1139; topk-moe.cu) ---------------
 __global__ void moe_route_kernel(const float* __restrict__ logits, int n_expert, int top_k, int* __restrict__ ids, float* __restrict__ w) {
@@ -1161,12 +1375,13 @@ int gemv(const GemvParams& p_in, int wtype, cudaStream_t stream) {
     if (use_qv3 < 0) { const char* e = getenv("DLP_GEMV_QV3"); use_qv3 = (e && e[0] == '0') ? 0 : 1; }
     if (use_qv3 && (wtype == W_Q8_0 || wtype == W_Q4_K || wtype == W_Q5_K || wtype == W_Q6_K)) {
         const size_t xsm = (size_t)T * K * 2 + ar_stage_bytes(p.ar_in.buf != nullptr, T, K);
-        int rc = -2;
+        int rc = wtype == W_Q6_K ? launch_gemv_q6_ring(p, stream) : -2;
+        if (rc != -2) return rc;
 #define DLP_QV3(WT_)                                                                                       \
     case WT_:                                                                                              \
-        rc = T == 1 ? launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 1>, p, xsm, stream, QChunkW<WT_>::value)   \
-           : T == 2 ? launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 2>, p, xsm, stream, QChunkW<WT_>::value)   \
-                    : launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 4>, p, xsm, stream, QChunkW<WT_>::value);  \
+        rc = T == 1 ? launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 1>, p, xsm, stream, QChunkW<WT_>::value, WT_ == W_Q4_K || WT_ == W_Q5_K)   \
+           : T == 2 ? launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 2>, p, xsm, stream, QChunkW<WT_>::value, WT_ == W_Q4_K || WT_ == W_Q5_K)   \
+                    : launch_gemv_qv3(gemv_quant_v3_kernel<WT_, 4>, p, xsm, stream, QChunkW<WT_>::value, WT_ == W_Q4_K || WT_ == W_Q5_K);  \
         break;
         switch (wtype) { DLP_QV3(W_Q8_0) DLP_QV3(W_Q4_K) DLP_QV3(W_Q5_K) DLP_QV3(W_Q6_K) }
 #undef DLP_QV3

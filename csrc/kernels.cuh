@@ -155,6 +155,7 @@ int gemm_quant_pieces(const QWeight& w0, const QWeight* w1, int wtype, const voi
 // *out |= 1 when a bounded wait of the named kernels has run out on the current device since the library was loaded
 int gemm_pair_expired(int* out);
 int gemm_quant_small_expired(int* out);
+int gemv_expired(int* out);
 int attn_prefill_expired(int* out);
 // MoE routing plan + data movement around the grouped GEMMs (moe.cu)
 int moe_route_ex(const float* logits, int ld, int T, int n_expert, int top_k, int renorm, int* ids, float* w, cudaStream_t s);

@@ -85,7 +85,7 @@ class LlamaEngine(EngineCore):
             self.comm.reserve_logits(max_seqs, v1 - v0, f32, dev)     # before any graph is captured
         # splits of the cached keys by batch size (index: queries of the step)
         n_sm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 0
-        self.attn_splits = [0] + [attn_splits if attn_splits is not None else ops.attn_splits(b, self.Hkv, self.Hq // self.Hkv, n_sm) if n_sm else 1
+        self.attn_splits = [0] + [attn_splits if attn_splits is not None else ops.attn_splits(b, self.Hkv, self.Hq // self.Hkv, n_sm, n_ctx) if n_sm else 1
                                   for b in range(1, max_seqs + 1)]
         parts = max(b * ns for b, ns in enumerate(self.attn_splits)) * self.Hq
         self.attn_ws = (torch.zeros(parts * self.D, dtype=f32, device=dev), torch.zeros(parts * 2, dtype=f32, device=dev),

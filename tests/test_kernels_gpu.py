@@ -68,6 +68,25 @@ def test_gemv_fused_norm_and_swiglu(t):
     assert nmse(ref, y) < (2e-4 if t.name.startswith("Q") else 2e-5)
 
 
+@pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
+@pytest.mark.parametrize("T", [1, 2, 4])
+@pytest.mark.parametrize("N,K", [(2, 256), (298, 768), (1002, 2048), (3000, 5632), (640, 14336)])
+def test_gemv_quant_of_every_width(t, T, N, K):
+    """Fewer rows than blocks, one and several stages of the Q6_K ring of which the last is partial, columns that end inside a warp's round, widths at
+    which a stage holds 8 rows down to 1 - plain, with the residual add, and with norm and gate.  The activations are rounded to 8 bits (relative
+    to the largest of 32: squared error 2.5e-5 of randn values; the few sums of the smallest shapes scatter by a factor of 10 around it)."""
+    (w, exact), (u, exact_u) = _w(N, K, t, 1), _w(N, K, t, 2)
+    g = torch.Generator(DEV).manual_seed(N)
+    h, norm = torch.randn(T, K, device=DEV, generator=g), torch.rand(K, device=DEV, generator=g) + 0.5
+    x = (h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-5) * norm).half()
+    ref, up = x.double() @ exact.double().T, x.double() @ exact_u.double().T
+    tol = 5e-5 if N * T > 500 else 5e-4
+    assert nmse(ref, ops.linear(w, x, "f32")) < tol
+    assert nmse(ref + 1, ops.linear(w, x, "add", out=torch.ones(T, N, device=DEV))) < tol
+    assert nmse(ref, ops.linear(w, h, "f32", norm_w=norm, eps=1e-5)) < tol
+    assert nmse(torch.nn.functional.silu(ref) * up, ops.linear(w, h, "swiglu", w_up=u, norm_w=norm, eps=1e-5)) < 4 * tol
+
+
 @pytest.mark.parametrize("t", [GGMLType.F16, GGMLType.BF16])
 @pytest.mark.parametrize("T", [1, 2, 4])
 @pytest.mark.parametrize("N,K", [(6144, 1024), (4736, 2048), (3072, 3584)])
