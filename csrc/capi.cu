@@ -115,7 +115,7 @@ int dlp_gemm_sp(const dlp_weight* w0, const dlp_weight* w1, const void* x, int l
     const size_t ws_bytes = coll ? coll->ws_bytes : 0;
     const int sk = ws ? 0 : 1;     // with a workspace: automatic deterministic split-K for skinny shards
     if (wt == DLP_W_F16 || wt == DLP_W_BF16)
-        return gemm_f16(w0->base, w1 ? w1->base : nullptr, w0->K, x, ldx, y, ldy, T, w0->N, w0->K, epilogue, wt == DLP_W_BF16, sk, s,
+        return gemm_f16(w0->base, w1 ? w1->base : nullptr, w0->K, x, ldx, y, ldy, T, w0->N, w0->K, epilogue, wt == DLP_W_BF16, sk, true, s,
                         coll ? &c : nullptr, nullptr, ws, ws_bytes);
     const QWeight q0 = to_qw(w0);
     QWeight q1;
@@ -153,7 +153,7 @@ static int linear_impl(const dlp_weight* w0, const dlp_weight* w1, const void* x
     cudaStream_t s = (cudaStream_t)stream;
     if (wt == DLP_W_F16 || wt == DLP_W_BF16)
         return gemm_f16(w0->base, w1 ? w1->base : nullptr, w0->K, x, w0->K, y, ldy, T, w0->N, w0->K, epi,
-                        wt == DLP_W_BF16, 0, s, nullptr, nullptr, ws, ws_bytes);
+                        wt == DLP_W_BF16, 0, true, s, nullptr, nullptr, ws, ws_bytes);
     // block-quantised: for prompts pieces of the weights are unpacked to scratch and multiplied (gemm_quant_pieces), otherwise, or without
     // scratch, the decode is fused into the GEMM.  DLP_GEMM_DEQUANT_SCRATCH=1: the whole matrix to scratch at any size, for A/B runs.
     static int two_pass = -1;
@@ -177,7 +177,7 @@ static int linear_impl(const dlp_weight* w0, const dlp_weight* w1, const void* x
         rc = dequant_rows_f16(to_qw(w1), wt, nullptr, w1->N, (__half*)up, w1->K, s);
         if (rc) return rc;
     }
-    return gemm_f16(scratch, up, w0->K, x, w0->K, y, ldy, T, w0->N, w0->K, epi, 0, 0, s, nullptr, nullptr, ws, ws_bytes);
+    return gemm_f16(scratch, up, w0->K, x, w0->K, y, ldy, T, w0->N, w0->K, epi, 0, 0, false, s, nullptr, nullptr, ws, ws_bytes);
 }
 
 int dlp_linear(const dlp_weight* w0, const dlp_weight* w1, const void* x, const float* norm_w, float eps, void* y,
@@ -211,7 +211,7 @@ int dlp_linear_grouped(const dlp_weight* w0, const dlp_weight* w1, const void* x
     cudaStream_t s = (cudaStream_t)stream;
     if (wt == DLP_W_F16 || wt == DLP_W_BF16)
         return gemm_f16(w0->base, w1 ? w1->base : nullptr, w0->K, xs, w0->K, y, ldy, n_assign, rows_per_expert, w0->K, epi, wt == DLP_W_BF16,
-                        ws ? 0 : 1, s, nullptr, &g, ws, ws_bytes);
+                        ws ? 0 : 1, true, s, nullptr, &g, ws, ws_bytes);
     const QWeight q0 = to_qw(w0);
     QWeight q1;
     if (w1) q1 = to_qw(w1);

@@ -70,7 +70,7 @@ int dlp_set_trace(void* buf) { set_trace_buffer((unsigned long long*)buf); retur
 int dlp_gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, void* y, int ldy, int T, int N,
                  int K, int epilogue, int is_bf16, int split_k, void* stream) {
     DLP_REQUIRE(w0 && x && y, "dlp_gemm_f16: null argument");
-    return gemm_f16(w0, w1, ldw, x, ldx, y, ldy, T, N, K, epilogue, is_bf16, split_k, (cudaStream_t)stream);
+    return gemm_f16(w0, w1, ldw, x, ldx, y, ldy, T, N, K, epilogue, is_bf16, split_k, false, (cudaStream_t)stream);
 }
 
 int dlp_advance(int32_t* seq_len, const int32_t* active, int32_t* pos, int32_t* slot, int32_t* kv_len,

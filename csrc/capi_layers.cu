@@ -29,9 +29,9 @@ int dlp_layers_linear(const void* x, int ldx, const void* w, int ldw, int N, int
     if (f32) return sgemm((const float*)x, ldx, (const float*)w, ldw, N, K, out, ldo, out_mode, T, (cudaStream_t)stream, nullptr, tl);
     DLP_REQUIRE(!tl || (out_mode == LO_F32 && tl->n2 >= 0 && (tl->n2 >= N || (tl->out2 && tl->ldo2 >= N - tl->n2))), "dlp_layers_linear: what follows the sums");
     if (out_mode == LO_GEGLU || out_mode == LO_SWIGLU)       // rows 2i / 2i+1 of the interleaved matrix: two operands with twice the row stride
-        return gemm_f16(w, (const uint8_t*)w + (size_t)ldw * 2, 2 * ldw, x, ldx, out, ldo, T, N / 2, K, out_mode == LO_GEGLU ? 6 : 8, 1, 0, (cudaStream_t)stream, nullptr, nullptr, ws, ws_bytes);
+        return gemm_f16(w, (const uint8_t*)w + (size_t)ldw * 2, 2 * ldw, x, ldx, out, ldo, T, N / 2, K, out_mode == LO_GEGLU ? 6 : 8, 1, 0, true, (cudaStream_t)stream, nullptr, nullptr, ws, ws_bytes);
     DLP_REQUIRE(out_mode == LO_F32 || out_mode == LO_BF16 || out_mode == LO_RELU2, "dlp_layers_linear: output mode %d", out_mode);
-    return gemm_f16(w, nullptr, ldw, x, ldx, out, ldo, T, N, K, tl ? 9 : out_mode == LO_BF16 ? 4 : out_mode == LO_RELU2 ? 7 : 1, 1, 0, (cudaStream_t)stream, nullptr, nullptr, ws, ws_bytes,
+    return gemm_f16(w, nullptr, ldw, x, ldx, out, ldo, T, N, K, tl ? 9 : out_mode == LO_BF16 ? 4 : out_mode == LO_RELU2 ? 7 : 1, 1, 0, true, (cudaStream_t)stream, nullptr, nullptr, ws, ws_bytes,
                     tl);
 }
 int dlp_layers_head_matmul(const void* x, int x_f32, int ldx, int x_head, int kx, const void* w, int Kp, int H, int N, int n_rows, void* out, int ldo, int out_head,
@@ -101,10 +101,10 @@ int dlp_layers_linear_grouped(const void* xs, int ldx, const void* w, int ldw, i
     if (f32) return sgemm((const float*)xs, ldx, (const float*)w, ldw, rows_per_expert, K, out, ldo, out_mode, n_assign, (cudaStream_t)stream, &g);
     if (out_mode == LO_SWIGLU) {       // two operands with twice the row stride, as in dlp_layers_linear
         g.rows_per_expert = rows_per_expert / 2;
-        return gemm_f16(w, (const uint8_t*)w + (size_t)ldw * 2, 2 * ldw, xs, ldx, out, ldo, n_assign, rows_per_expert / 2, K, 8, 1, ws ? 0 : 1, (cudaStream_t)stream, nullptr, &g, ws,
+        return gemm_f16(w, (const uint8_t*)w + (size_t)ldw * 2, 2 * ldw, xs, ldx, out, ldo, n_assign, rows_per_expert / 2, K, 8, 1, ws ? 0 : 1, true, (cudaStream_t)stream, nullptr, &g, ws,
                         ws_bytes);
     }
-    return gemm_f16(w, nullptr, ldw, xs, ldx, out, ldo, n_assign, rows_per_expert, K, out_mode == LO_RELU2 ? 7 : 1, 1, ws ? 0 : 1, (cudaStream_t)stream, nullptr, &g, ws,
+    return gemm_f16(w, nullptr, ldw, xs, ldx, out, ldo, n_assign, rows_per_expert, K, out_mode == LO_RELU2 ? 7 : 1, 1, ws ? 0 : 1, true, (cudaStream_t)stream, nullptr, &g, ws,
                     ws_bytes);
 }
 int dlp_layers_combine(const float* y, int ldy, const int32_t* pos, const float* weights, int T, int top, int E, float* out, const float* ys, const float* gs, int ldgs,

@@ -57,7 +57,7 @@ int make_tmap_bytes(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
 
 // Y[T,N] (op)= X[T,K] . W0[N,K]^T  (and W1 for SwiGLU).  X/W are fp16 (is_bf16=0) or bf16 (is_bf16=1).
 int gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, void* y, int ldy, int T, int N, int K,
-             int epilogue, int is_bf16, int split_k, cudaStream_t stream, const GemmCollective* coll, const GemmGroup* grp, void* ws,
+             int epilogue, int is_bf16, int split_k, bool w_static, cudaStream_t stream, const GemmCollective* coll, const GemmGroup* grp, void* ws,
              size_t ws_bytes, const OutTail* tail) {
     // grouped: N = output features of ONE expert, w0/w1 = stacks of all experts (rows_total = what the tensor map must cover)
     DLP_REQUIRE(T > 0 && N > 0 && K > 0, "gemm: empty problem T=%d N=%d K=%d", T, N, K);
@@ -88,7 +88,7 @@ int gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, vo
     if (tail) p.tail = *tail;
     DLP_REQUIRE(epilogue != EPI_RS_PUSH_F32 || (coll && coll->rs_rows > 0 && coll->rs_done && coll->rs_tp >= 1 && coll->rs_tp <= 8 && splits == 1),
                 "gemm: the reduce-scatter epilogue needs a collective descriptor and no atomic split-K");
-    p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue;
+    p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue; p.w_static = w_static;
     if (grp) p.grp = *grp;
     if (coll == nullptr && split_k <= 1 && gemm_pair_takes(T, grp)) return gemm_pair(p, w0, w1, ldw, x, ldx, is_bf16, na, split_k, stream);
     const int bt = grp ? grp->bt : (T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256);

@@ -31,6 +31,7 @@ struct GemmParams {
     int ldy;       // row stride of y in elements
     int epilogue;
     int k_blocks_per_split;
+    bool w_static;         // the weights may be requested before the predecessor has finished (gemm_f16)
     GemmCollective coll;   // fused all-gather (X side) / reduce-scatter (Y side); zero-initialised = none
     GemmGroup grp;         // grouped (MoE) launch: per-tile expert / row range table built on the device
     // split-K with a deterministic fix-up (any epilogue): every split stores its fp32 partial tile into `ws`, the split that
@@ -295,9 +296,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     int t0 = blockIdx.y * BT;           // first token row (B operand, output row)
     int t_end = p.T;                    // output rows >= t_end are not stored
     const int n_out0 = n0;              // first output column
-    // Weights are static: in a plain launch the first stages of them are requested, and barriers and tensor memory set up, while the predecessor
-    // still runs.  Everything else waits for it: the tokens, what a collective or the table of a grouped launch says, and the epilogue.
-    const bool ahead = p.grp.tile_expert == nullptr && p.coll.x_flags == nullptr;
+    // Static weights: in a plain launch the first stages of them are requested, and barriers and tensor memory set up, while the predecessor
+    // still runs.  Everything else waits for it, an operand that the predecessor makes included: the tokens, what a collective or the table of a grouped launch says, and the epilogue.
+    const bool ahead = p.w_static && p.grp.tile_expert == nullptr && p.coll.x_flags == nullptr;
     if (!ahead) pdl_wait();
     if (p.grp.tile_expert != nullptr) {
         // grouped launch: this token tile belongs to one expert; its weight rows sit at expert * rows_per_expert in the stack

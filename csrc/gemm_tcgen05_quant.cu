@@ -57,7 +57,8 @@ int gemm_quant_pieces(const QWeight& w0, const QWeight* w1, int wtype, const voi
             default: DLP_REQUIRE(false, "gemm_quant: unsupported weight type %d", wtype);
         }
         const size_t size = epilogue == EPI_STORE_F16 || epilogue == EPI_SWIGLU_F16 ? 2 : 4;
-        const int rc = gemm_f16(out, na == 2 ? out + (size_t)rows * K : nullptr, K, x, K, (uint8_t*)y + (size_t)n0 * size, ldy, T, rows, K, epilogue, 0, 0, stream);
+        // (the launch before this one makes the operand: not static)
+        const int rc = gemm_f16(out, na == 2 ? out + (size_t)rows * K : nullptr, K, x, K, (uint8_t*)y + (size_t)n0 * size, ldy, T, rows, K, epilogue, 0, 0, false, stream);
         if (rc) return rc;
     }
     return 0;
@@ -92,7 +93,7 @@ int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, i
     if (coll) p.coll = *coll;
     DLP_REQUIRE(epilogue != EPI_RS_PUSH_F32 || (coll && coll->rs_rows > 0 && coll->rs_done && coll->rs_tp >= 1 && coll->rs_tp <= 8 && splits == 1),
                 "gemm: the reduce-scatter epilogue needs a collective descriptor and no atomic split-K");
-    p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue;
+    p.y = y; p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.epilogue = epilogue; p.w_static = true;
     if (grp) p.grp = *grp;
     int bt = grp ? grp->bt : (T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256);
     const QWeight up = w1 ? *w1 : QWeight();

@@ -143,8 +143,10 @@ struct OutTail {
 };
 
 int gemv(const GemvParams& p, int wtype, cudaStream_t stream);
+// w_static: no launch still at work in the stream writes w0 / w1 (weights of a model), so that they may be requested before the predecessor has
+// finished; false for an operand that a launch before this one makes (unpacked weights)
 int gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, void* y, int ldy, int T, int N, int K,
-             int epilogue, int is_bf16, int split_k, cudaStream_t stream, const GemmCollective* coll = nullptr,
+             int epilogue, int is_bf16, int split_k, bool w_static, cudaStream_t stream, const GemmCollective* coll = nullptr,
              const GemmGroup* grp = nullptr, void* ws = nullptr, size_t ws_bytes = 0, const OutTail* tail = nullptr);
 int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, int ldx, void* y, int ldy, int T, int epilogue,
                int split_k, cudaStream_t stream, const GemmCollective* coll = nullptr, const GemmGroup* grp = nullptr, void* ws = nullptr,

@@ -52,12 +52,15 @@ int dlp_set_trace(void* buf);
 
 /* Decode mat-vec, T in {1,2,4}: y[T,N] (op)= x[T,K] . W^T.  If norm_w != NULL, x is the fp32 residual stream and
  * RMSNorm(x)*norm_w is fused into the prologue; otherwise x is fp16.  out_mode SWIGLU takes w0=gate, w1=up.
+ * Here and wherever a call takes a dlp_weight: the matrix is that of a model, requested while the launch before this one still runs, so
+ * no kernel of this library that directly precedes the call in the stream may write it (unpacked rows go to dlp_gemm_f16).
  * ref: mul_mat_vec_f / mul_mat_vec_q + GLU fusion (ggml-cuda/mmvf.cu, mmvq.cu:143,181-189). */
 int dlp_gemv(const dlp_weight* w0, const dlp_weight* w1, const void* x, const float* norm_w, float eps, void* y,
              int ldy, int out_mode, int T, void* stream);
 
 /* tcgen05/TMEM/TMA GEMM on dense fp16 (is_bf16=0) or bf16 operands: y[T,N] (op)= x[T,K] . w0[N,K]^T.
  * epilogue: 0 store f16, 1 store f32, 2 atomic-add f32 (allows split_k>1; 0 = auto), 3 SwiGLU f16 (w1 = up), 4 store bf16.
+ * Any launch before this one in the stream may write w0, w1 and x.
  * ref: cuBLAS GemmEx fallback + mma.sync MMQ (ggml-cuda/ggml-cuda.cu:1227-1371, mmq.cuh:3459). */
 int dlp_gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx, void* y, int ldy, int T, int N,
                  int K, int epilogue, int is_bf16, int split_k, void* stream);

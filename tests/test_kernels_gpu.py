@@ -223,6 +223,56 @@ def test_linear_quant_two_pass_scratch_entry_point():
     assert rc == 0 and nmse(x.float() @ exact.T, y) < 5e-6
 
 
+def test_products_with_an_operand_unpacked_just_before():
+    """Rows unpacked by one launch are the weights of the next, which may be requested early only where nothing writes them: different weights through
+    one buffer, back to back, against 64 bits (fp16 values, fp32 sums)."""
+    N, K, T = 384, 2048, (3, 5, 16, 17, 64, 65, 300)
+    ws = [_w(N, K, t, i) for i, t in enumerate((GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q6_K))]
+    buf = torch.full((N, K), math.nan, dtype=torch.float16, device=DEV)
+    xs = [torch.randn(t, K, device=DEV, generator=torch.Generator(DEV).manual_seed(t)).half() for t in T]
+    cases = [(x, w, x.double() @ exact.half().double().T, torch.zeros(len(x), N, device=DEV)) for x in xs for _ in range(3) for w, exact in ws]
+    for x, w, _, y in cases:
+        ops.dequant_rows(w, None, out=buf)
+        ops.gemm_f16(buf, x, y, epilogue=1)
+    assert max(nmse(ref, y) for _, _, ref, y in cases) < 1e-11
+
+
+_WHOLE_MATRIX_UNPACKED = """
+import ctypes as C, sys, torch
+sys.path.insert(0, "tests")
+from test_kernels_gpu import _w, nmse, ops, GGMLType
+from distributed_llm_pipeline_b200.ops import lib as L
+assert ops.TWO_PASS_DEQUANT
+N, K = 384, 1024
+(a, ea), (b, eb) = _w(N, K, GGMLType.Q4_K, 1), _w(N, K, GGMLType.Q8_0, 2)
+scratch = torch.full((N * K * 2,), float("nan"), dtype=torch.float16, device="cuda").view(torch.uint8)
+for T in (3, 5, 16, 64, 100):
+    x = torch.randn(T, K, device="cuda").half()
+    ra, rb = x.double() @ ea.double().T, x.double() @ eb.double().T
+    silu = torch.nn.functional.silu
+    for _ in range(3):
+        ys = []
+        for w, u in ((a, None), (b, None), (b, b), (a, a)):
+            y = torch.zeros(T, N, device="cuda", dtype=torch.float16 if u else torch.float32)
+            rc = L.load().dlp_linear(w.ref(), u.ref() if u else None, x.data_ptr(), None, 0.0, y.data_ptr(), N, 3 if u else 1, T, scratch.data_ptr(), scratch.numel(),
+                                     torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+            ys.append(y)
+        for y, ref in zip(ys, (ra, rb, silu(rb) * rb, silu(ra) * ra)):
+            assert nmse(ref, y) < 2e-6, T
+print("ok")
+"""
+
+
+def test_whole_matrix_unpacked_to_scratch():
+    """DLP_GEMM_DEQUANT_SCRATCH=1 (read once a process): weights that share one scratch, one call after the other, with and without a gate."""
+    import os
+    import subprocess
+    import sys
+    res = subprocess.run([sys.executable, "-c", _WHOLE_MATRIX_UNPACKED], capture_output=True, text=True, timeout=300, env={**os.environ, "DLP_GEMM_DEQUANT_SCRATCH": "1", "PYTHONPATH": "."})
+    assert res.returncode == 0 and "ok" in res.stdout, res.stdout + res.stderr
+
+
 def test_rmsnorm_with_residual():
     T, E = 7, 1024
     h = torch.randn(T, E, device=DEV)
