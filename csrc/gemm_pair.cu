@@ -43,7 +43,7 @@ static int launch_pair(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUt
 
 int gemm_pair(const GemmParams& p, const void* w0, const void* w1, int ldw, const void* x, int ldx, int is_bf16, int na, int split_k, cudaStream_t stream) {
     const GemmGroup* grp = p.grp.tile_expert ? &p.grp : nullptr;
-    const PairPlan pl = pair_plan(p.T, p.N, p.K, na, p.epilogue == EPI_ATOMIC_ADD_F32 && split_k <= 0, grp);
+    const PairPlan pl = pair_plan(p.T, p.N, p.K, na, p.epilogue == EPI_ATOMIC_ADD_F32 && split_k <= 0 && gemm_add_may_split(p.T, p.N, (p.K + GEMM_BK - 1) / GEMM_BK), grp);
     const uint64_t w_rows = grp ? (uint64_t)grp->rows_per_expert * grp->n_expert : (uint64_t)p.N;
     CUtensorMap tw0, tw1, tx;
     int rc;

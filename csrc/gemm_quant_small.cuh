@@ -362,21 +362,23 @@ static int launch_quant_small(const QWeight& w0, const QWeight& w1, const CUtens
     const int units = p.K / Cfg::COLS;
     const long tiles_n = (p.N + GEMM_BM - 1) / GEMM_BM, tiles_t = p.grp.tile_expert ? p.grp.max_tiles : (p.T + BT - 1) / BT, tiles = tiles_n * tiles_t;
     int splits = split_k > 0 ? split_k : 1;
+    bool by_ws = false;
     p.ws = nullptr;
     p.ws_counters = nullptr;
-    if (split_k <= 0 && p.epilogue == EPI_ATOMIC_ADD_F32) splits = quant_small_splits(tiles, units, sm_count() * Cfg::PER_SM);
+    if (split_k <= 0 && p.epilogue == EPI_ATOMIC_ADD_F32 && gemm_add_may_split(p.T, p.N, p.K / GEMM_BK)) splits = quant_small_splits(tiles, units, sm_count() * Cfg::PER_SM);
     else if (split_k <= 0 && ws != nullptr && tiles <= (long)GEMM_WS_COUNTERS && p.epilogue != EPI_RS_PUSH_F32) {
         // (grouped: the table decides how many tiles there are; most routings of few tokens fill about half of the bound)
         splits = quant_small_splits(p.grp.tile_expert ? (tiles + 1) / 2 : tiles, units, sm_count() * Cfg::PER_SM);
         if (splits > 8) splits = 8;
         const size_t per = (size_t)NA * BT * GEMM_BM * sizeof(float);
         while (splits > 1 && GEMM_WS_COUNTERS * 4 + (size_t)tiles * splits * per > ws_bytes) --splits;
+        by_ws = true;
     }
     if (splits > units) splits = units;
     const int per_split = (units + splits - 1) / splits;
     splits = (units + per_split - 1) / per_split;
     p.k_blocks_per_split = per_split * Cfg::SLICES;
-    if (splits > 1 && p.epilogue != EPI_ATOMIC_ADD_F32) {
+    if (splits > 1 && by_ws) {
         p.ws_counters = reinterpret_cast<unsigned*>(ws);
         p.ws = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + GEMM_WS_COUNTERS * 4);
     }

@@ -461,6 +461,12 @@ static int launch_gemm(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUt
 // a fraction of the HBM rate.  Workspace layout: 4096 tile counters (zero-initialised by the owner, self-resetting), then
 // [tile][split][accumulator][BT][128] fp32 partials.
 constexpr size_t GEMM_WS_COUNTERS = 4096;
+// Whether the residual epilogue may be split over K with atomics, whose order - and with it the last bits of the sums - changes from run to run:
+// only where tiles of 128 features would leave half of the SMs idle.  All other products repeat themselves exactly.
+static inline bool gemm_add_may_split(int T, int N, int total_kb) {
+    const int bt = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
+    return (long)((N + GEMM_BM - 1) / GEMM_BM) * ((T + bt - 1) / bt) * 2 <= sm_count() && total_kb / 2 >= 8;
+}
 static int auto_split_ws(int epilogue, int split_k, long tiles, int total_kb, int na, int bt, void* ws, size_t ws_bytes, GemmParams& p) {
     // Measured (profiles/r2_gemm_splitk_ab.txt): the fix-up pays for token tiles up to 32 (decode batches: +19 % at B = 8); for
     // prefill-sized tiles the serial reload of 128 x 256 partials costs more than the idle SMs (54 k -> 29 k tok/s at pp512), and

@@ -194,6 +194,20 @@ def test_linear_quant_few_tokens(t, T, N, K):
     assert nmse(torch.nn.functional.silu(ref) * (x.double() @ exact_u.double().T), ops.linear(w, x, "swiglu", w_up=u)) < 2e-6
 
 
+@pytest.mark.parametrize("T,N,K,t", [(553, 4096, 4096, GGMLType.F16), (1041, 2048, 5632, GGMLType.F16), (1041, 4096, 4096, GGMLType.Q8_0), (7, 9600, 1536, GGMLType.Q4_K),
+                                     (40, 2048, 512, GGMLType.Q8_0), (150, 9600, 768, GGMLType.Q6_K)])
+def test_residual_sums_repeat(T, N, K, t):
+    """Sizes at which the tiles fill the machine: the residual add gives the same bits every time (no atomics of several splits of K), also through the
+    workspace, and is right."""
+    w = DeviceWeight.from_dense(torch.randn(N, K, generator=torch.Generator().manual_seed(1)) * 0.05, t, DEV)
+    x = torch.randn(T, K, device=DEV, generator=torch.Generator(DEV).manual_seed(T)).half()
+    base = torch.randn(T, N, device=DEV, generator=torch.Generator(DEV).manual_seed(N))
+    runs = [ops.linear(w, x, "add", out=base.clone()) for _ in range(10)]
+    assert all(torch.equal(runs[0], r) for r in runs)
+    dense = ops.dequant_rows(w, None, out=torch.empty(N, K, device=DEV)) if t.name.startswith("Q") else w.planes[0].view(N, K)
+    assert nmse(base.double() + x.double() @ dense.double().T, runs[0]) < 2e-7
+
+
 @pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
 @pytest.mark.parametrize("T,N,K,kib", [(193, 256, 256, 256), (300, 700, 512, 512), (1025, 1280, 768, 1 << 16)])
 def test_linear_quant_prompt_in_pieces(t, T, N, K, kib):
