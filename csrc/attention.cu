@@ -43,12 +43,17 @@ __device__ __forceinline__ uint32_t movmatrix(uint32_t a) {      // 8 x 8 halves
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
     return d;
 }
-// two fp32 values as fp16 pairs: value and remainder (22 bits together)
-__device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_t& lo) {
+// two fp32 values as fp16 pairs: value and remainder (23 bits together), or with `rest` what is left of those as well (all 24)
+__device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_t& lo, uint32_t* rest = nullptr) {
     const __half2 h = __floats2half2_rn(a, b);
     const float2 f = __half22float2(h);
     hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = pack_h2(a - f.x, b - f.y);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+    if (rest != nullptr) {
+        const float2 g = __half22float2(l);
+        *rest = pack_h2((a - f.x) - g.x, (b - f.y) - g.y);
+    }
 }
 
 // ---- split-KV attention on the tensor cores ------------------------------------------------------------------------------
@@ -57,8 +62,12 @@ __device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_
 // K / V byte is read once.  (Heads as the 16 rows: half of the tile is padding, twice the MMAs.)  Each of the 4 warps streams its own tiles of 16 keys through a private ring of
 // 3 stages (cp.async, 8 KB a stage at D = 128; 2 CTAs an SM: 128 KB in flight) and keeps its own running maximum; page ids are fetched one
 // tile ahead; the warps are merged through shared memory, the splits by the last CTA of the (query, head) to finish.
-// Scores and sums are fp32; the softmax weights (and with ROPE the rotated fp32 queries) enter the tensor cores as two fp16 parts, value and
-// remainder, in units of 2^-10 so that the remainder of small weights is not lost to subnormals.
+// Scores and sums are fp32.  The softmax weights (and with ROPE the rotated fp32 queries) enter the tensor cores as two (three) fp16 parts, value
+// and remainder, 23 (24) bits together, scaled by powers of two so that no part overflows or goes subnormal where it counts: weights in units of
+// 2^-15, a head's queries by its largest one.  What an MMA adds is cut off, not rounded, at the size of its largest term, so no MMA adds to a
+// sum that is kept: each takes 16 products from zero, parts apart, and the sums over them are rounded fp32 additions.  Error against 64 bits
+// before the output's rounding, 32 heads over 8, D = 128, keys of deviation 1.5: 700 keys 2.4e-7 (fp32 FMA per key 2.4e-7, sums kept in the MMAs
+// 4.1e-7), 32,000 3.1e-7 (3.4e-7, 8.3e-7).
 // 32,000 keys of 8 KV heads of 4 query heads, D = 128 (131 MB): 28.5 us (4.6 TB/s; 108 us with fp32 FMA per key in 128 CTAs); 32 queries
 // of up to 2,000 keys (135 MB): 34 us (117 us).
 //   ROPE: takes the fp32 row of the QKV mat-vec, rotates q in registers, writes the new token's K and V and uses them from shared memory.
@@ -85,10 +94,11 @@ struct AttnRope {
 };
 
 // One warp joins the partials of `eff` splits of one (query, head): a lane takes D / 32 dims, its loads of 8 splits in flight at a time.
-// (Maxima are in units of log 2.  One thread per dim, splits one after the other: 45 us instead of 28.5 for 32,000 keys in 37 splits.)
+// (One thread per dim, splits one after the other: 45 us instead of 28.5 for 32,000 keys in 37 splits.)
 template <int D>
 __device__ __forceinline__ void attn_join(const AttnParams& p, size_t head, int eff, int lane) {
     constexpr int E = D / 32;
+    constexpr float LOG2E = 1.4426950408889634f;
     const size_t pi0 = head * p.n_splits;
     const float* ml = p.part_ml + pi0 * 2;
     float mn = -INFINITY, ls = 0.f, acc[E];
@@ -98,7 +108,7 @@ __device__ __forceinline__ void attn_join(const AttnParams& p, size_t head, int 
     mn = warp_max(mn);
     for (int s0 = 0; s0 < eff; s0 += 32) {
         const float2 v = s0 + lane < eff ? make_float2(__ldcg(ml + 2 * (s0 + lane)), __ldcg(ml + 2 * (s0 + lane) + 1)) : make_float2(-INFINITY, 0.f);
-        const float a = v.x == -INFINITY ? 0.f : exp2f(v.x - mn);
+        const float a = v.x == -INFINITY ? 0.f : exp2f((v.x - mn) * LOG2E);
         ls += v.y * a;
         const int n = min(32, eff - s0);
         for (int s = 0; s < n; s += 8) {
@@ -128,7 +138,7 @@ template <int D> constexpr int attn_split_smem() { return 4 * 3 * 2 * 16 * D * 2
 template <int D, int NH, bool ROPE>      // NH: groups of 8 query heads in use
 __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, const AttnRope ra) {
     constexpr int STAGES = 3, KS = D / 16, CPR = D / 8, TILE = 16 * D * 2;      // k steps, 16-byte chunks per row, bytes of one K or V tile
-    constexpr float LOG2E = 1.4426950408889634f, UP = 10.f;
+    constexpr float LOG2E = 1.4426950408889634f, UP = 32768.f;
     extern __shared__ __align__(128) uint8_t as_smem[];
     const int gqa = p.Hq / p.Hkv, R = 8 * NH, groups = (gqa + R - 1) / R;
     const int kvh = blockIdx.y / groups, h0 = (blockIdx.y % groups) * R, G = min(R, gqa - h0), hq0 = kvh * gqa + h0;
@@ -174,7 +184,8 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
     trace_event(p.trace, TR_ATTN | TR_WAITED);
 
     // queries as B fragments: head g, dims ks * 16 + 2t, + 1 and + 8, + 9
-    uint32_t qh[KS][NH][2], ql[ROPE ? KS : 1][NH][2];
+    uint32_t qh[KS][NH][2], ql[ROPE ? KS : 1][NH][2], qr[ROPE ? KS : 1][NH][2];
+    float unscale[NH][2];                    // ROPE: what brings the scores of heads 2t and 2t + 1 back to the queries' own size (a power of two)
     const float2* cs_tab = ROPE && ra.cs ? ra.cs + (size_t)qi * (D / 2) : nullptr;
     auto angle = [&](int i) {               // (cos, sin) of pair i
         if (cs_tab) return cs_tab[i];
@@ -211,13 +222,25 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
                         x[ks][e] = make_float2(u.x * a.x - u.y * a.y, u.x * a.y + u.y * a.x);
                     }
             }
+            float top = 0.f;
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const float sc = r < G ? ra.q_scale : 0.f;
-                    split_h2(x[ks][e].x * sc, x[ks][e].y * sc, qh[ks][nh][e], ql[ks][nh][e]);
+                    x[ks][e] = make_float2(x[ks][e].x * sc, x[ks][e].y * sc);
+                    top = fmaxf(top, fmaxf(fabsf(x[ks][e].x), fabsf(x[ks][e].y)));
                 }
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const int up = top > 0.f ? max(-100, min(100, 141 - (int)(__float_as_uint(top) >> 23))) : 0;      // the head's largest |q|: 2^14 .. 2^15
+            const float f = __uint_as_float((uint32_t)(127 + up) << 23), back = __uint_as_float((uint32_t)(127 - up) << 23);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) unscale[nh][h] = __shfl_sync(0xffffffffu, back, (2 * t + h) * 4);
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) split_h2(x[ks][e].x * f, x[ks][e].y * f, qh[ks][nh][e], ql[ks][nh][e], &qr[ks][nh][e]);
         } else {
             const __half* src = p.q + ((size_t)qi * p.Hq + hq0 + min(r, G - 1)) * D;
 #pragma unroll
@@ -285,12 +308,14 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
             }
             __syncwarp();
         }
-        constexpr int CHAINS = ROPE ? 4 : 2;      // independent accumulators: an MMA waits for the one before it in its chain
-        float s[NH][CHAINS][4];
+        // scores: keys g (0, 1) and g + 8 (2, 3), heads 2t (even) and 2t + 1; `low`: of the queries' remainders, 2^-12 of the others (what is cut off
+        // there does not count), in independent chains, since an MMA waits for the one before it in its chain
+        constexpr int CHAINS = NH == 1 ? 2 : 1;
+        float part[NH][KS / 2][4], low[NH][2 * CHAINS][4];
 #pragma unroll
         for (int nh = 0; nh < NH; ++nh)
 #pragma unroll
-            for (int c = 0; c < CHAINS; ++c) { s[nh][c][0] = s[nh][c][1] = s[nh][c][2] = s[nh][c][3] = 0.f; }
+            for (int c = 0; c < 2 * CHAINS; ++c) { low[nh][c][0] = low[nh][c][1] = low[nh][c][2] = low[nh][c][3] = 0.f; }
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
             uint32_t ka[4];
@@ -298,21 +323,38 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
             ldmatrix_x4(ka, sK + kr * (D * 2) + ((c ^ (kr & 7)) << 4));
 #pragma unroll
             for (int nh = 0; nh < NH; ++nh) {
-                mma_16816(s[nh][ks & 1], ka, qh[ks][nh][0], qh[ks][nh][1]);
-                if constexpr (ROPE) mma_16816(s[nh][2 + (ks & 1)], ka, ql[ks][nh][0], ql[ks][nh][1]);
+                float x[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_16816(x, ka, qh[ks][nh][0], qh[ks][nh][1]);
+                if constexpr (ROPE) {
+                    mma_16816(low[nh][ks % CHAINS * 2], ka, ql[ks][nh][0], ql[ks][nh][1]);
+                    mma_16816(low[nh][ks % CHAINS * 2 + 1], ka, qr[ks][nh][0], qr[ks][nh][1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[nh][ks / 2][e] = ks & 1 ? part[nh][ks / 2][e] + x[e] : x[e];
             }
         }
+#pragma unroll
+        for (int n = KS / 4; n >= 1; n /= 2)
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                for (int i = 0; i < n; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) part[nh][i][e] += part[nh][i + n][e];
         uint32_t ph[NH][2], pl[NH][2];       // weights as B fragments: head g, keys 2t, 2t + 1 and + 8, + 9
         float alpha[NH][2];
-        bool grew = false;
 #pragma unroll
         for (int nh = 0; nh < NH; ++nh) {
-            float v[4], pr[4];               // keys g (0, 1) and g + 8 (2, 3), heads 2t (even) and 2t + 1
+            float v[4], pr[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                float x = s[nh][0][e] + s[nh][1][e];
-                if constexpr (ROPE) x += s[nh][2][e] + s[nh][3][e];
-                v[e] = tok0 + g + (e >> 1) * 8 < rg.end ? x * LOG2E : -INFINITY;
+                float x = part[nh][0][e];
+                if constexpr (ROPE) {
+                    float y = low[nh][0][e] + low[nh][1][e];
+                    if constexpr (CHAINS == 2) y += low[nh][2][e] + low[nh][3][e];
+                    x = (x + y) * unscale[nh][e & 1];
+                }
+                v[e] = tok0 + g + (e >> 1) * 8 < rg.end ? x : -INFINITY;
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -320,29 +362,20 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                const float mn = fmaxf(m[nh][h], mx), off = mn == -INFINITY ? 0.f : mn - UP;
-                alpha[nh][h] = m[nh][h] == -INFINITY ? 0.f : exp2f(m[nh][h] - mn);
-                grew = grew || alpha[nh][h] != 1.f;
+                const float mn = fmaxf(m[nh][h], mx), off = mn == -INFINITY ? 0.f : mn;
+                alpha[nh][h] = m[nh][h] == -INFINITY ? 0.f : exp2f((m[nh][h] - mn) * LOG2E);
                 m[nh][h] = mn;
-                pr[h] = exp2f(v[h] - off);
-                pr[2 + h] = exp2f(v[2 + h] - off);
+                pr[h] = exp2f((v[h] - off) * LOG2E);
+                pr[2 + h] = exp2f((v[2 + h] - off) * LOG2E);
                 l[nh][h] = l[nh][h] * alpha[nh][h] + (pr[h] + pr[2 + h]);
             }
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 uint32_t hi, lo;
-                split_h2(pr[2 * e], pr[2 * e + 1], hi, lo);
+                split_h2(pr[2 * e] * UP, pr[2 * e + 1] * UP, hi, lo);
                 ph[nh][e] = movmatrix(hi);
                 pl[nh][e] = movmatrix(lo);
             }
-        }
-        if (__any_sync(0xffffffffu, grew)) {
-#pragma unroll
-            for (int i = 0; i < D / 16; ++i)
-#pragma unroll
-                for (int nh = 0; nh < NH; ++nh)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[i][nh][e] *= alpha[nh][e & 1];
         }
 #pragma unroll
         for (int i = 0; i < D / 16; ++i) {
@@ -351,8 +384,11 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
             ldmatrix_x4_trans(va, sV + vr * (D * 2) + ((c ^ (vr & 7)) << 4));
 #pragma unroll
             for (int nh = 0; nh < NH; ++nh) {
-                mma_16816(o[i][nh], va, ph[nh][0], ph[nh][1]);
-                mma_16816(o[i][nh], va, pl[nh][0], pl[nh][1]);
+                float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_16816(hi, va, ph[nh][0], ph[nh][1]);
+                mma_16816(lo, va, pl[nh][0], pl[nh][1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[i][nh][e] = fmaf(o[i][nh][e], alpha[nh][e & 1], hi[e] + lo[e]);
             }
         }
         __syncwarp();
@@ -376,8 +412,8 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
 #pragma unroll
                 for (int i = 0; i < D / 16; ++i) {
                     float* dst = sm_o + ((size_t)warp * R + r) * D + i * 16 + g;
-                    dst[0] = o[i][nh][h];
-                    dst[8] = o[i][nh][2 + h];
+                    dst[0] = o[i][nh][h] * (1.f / UP);
+                    dst[8] = o[i][nh][2 + h] * (1.f / UP);
                 }
                 if (g == 0) { sm_ml[(warp * R + r) * 2] = m[nh][h]; sm_ml[(warp * R + r) * 2 + 1] = ls; }
             }
@@ -390,7 +426,7 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
         for (int w = 0; w < 4; ++w) mn = fmaxf(mn, sm_ml[(w * R + r) * 2]);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const float mw = sm_ml[(w * R + r) * 2], a = mw == -INFINITY ? 0.f : exp2f(mw - mn);
+            const float mw = sm_ml[(w * R + r) * 2], a = mw == -INFINITY ? 0.f : exp2f((mw - mn) * LOG2E);
             acc += sm_o[((size_t)w * R + r) * D + d] * a;
             ls += sm_ml[(w * R + r) * 2 + 1] * a;
         }

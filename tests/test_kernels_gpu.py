@@ -483,6 +483,63 @@ def test_attn_split_tiles_and_joins(D, Hq, Hkv, page, n_splits):
     assert int(ws[2].abs().sum()) == 0
 
 
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 32, 8), (64, 32, 4), (128, 24, 2)])
+def test_attn_split_arithmetic_is_fp32(D, Hq, Hkv):
+    """Sums that cancel show what decode attention rounds: keys with values + 1024, others, and the first keys again with - 1024.  Each rounding of an fp32 sum of
+    that size is 2^-24 / sqrt(3) of it (rms); kept in the tensor cores' sums, which cut off, the error was 0.9 to 1.0 of 2^-24."""
+    page, n, err = 64, 300, {}
+    for rope in (False, True):
+        for seed in range(4):
+            g = torch.Generator(DEV).manual_seed(seed)
+            T = 3 * n
+            per = (T + page) // page
+            k, other = ((torch.randn(Hkv, n, D, device=DEV, generator=g) * 0.3) for _ in range(2))
+            big = torch.full((Hkv, n, D), 1024.0, device=DEV)
+            K = torch.cat([k, other, k], 1).half()
+            V = torch.cat([big, torch.randn(Hkv, n, D, device=DEV, generator=g), -big], 1).half()
+            kc, vc = torch.zeros(2, per, Hkv, page, D, device=DEV, dtype=torch.float16)
+            for cache, rows in ((kc, K), (vc, V)):
+                flat = torch.zeros(Hkv, per * page, D, device=DEV, dtype=torch.float16)
+                flat[:, :T] = rows
+                cache.copy_(flat.view(Hkv, per, page, D).permute(1, 0, 2, 3))
+            bt = torch.arange(per, dtype=torch.int32, device=DEV)[None].contiguous()
+            ws = (torch.zeros(Hq * 16 * D, device=DEV), torch.zeros(Hq * 32, device=DEV), torch.zeros(Hq, dtype=torch.int32, device=DEV))
+            if rope:            # (angles 0; the new token's own value is 0)
+                qkv = torch.randn(1, (Hq + 2 * Hkv) * D, device=DEV, generator=g)
+                qkv[:, (Hq + Hkv) * D:] = 0
+                out = ops.attn_decode_rope(qkv, torch.zeros(D // 2, device=DEV), kc, vc, bt, torch.tensor([T + 1], dtype=torch.int32, device=DEV), Hq, Hkv, D, n_splits=16, workspace=ws)
+                q = qkv.double().view(-1, D)[:Hq] * torch.tensor(D ** -0.5, dtype=torch.float32).double().item()
+                K, V = torch.cat([K, qkv.view(-1, D)[Hq:Hq + Hkv, None].half()], 1), torch.cat([V, torch.zeros_like(V[:, :1])], 1)
+            else:
+                q = (torch.randn(1, Hq * D, device=DEV, generator=g) * D ** -0.5).half()
+                out = ops.attn_paged(q, kc, vc, bt, torch.tensor([T], dtype=torch.int32, device=DEV), Hq, Hkv, D, n_splits=16, workspace=ws)
+                q = q.double().view(Hq, D)
+            p = torch.softmax(torch.einsum("hd,hnd->hn", q, K.double().repeat_interleave(Hq // Hkv, 0)), -1)
+            V = V.double().repeat_interleave(Hq // Hkv, 0)
+            e = (out.double().view(Hq, D) - torch.einsum("hn,hnd->hd", p, V)) / torch.einsum("hn,hnd->hd", p, V.abs())
+            err.setdefault(rope, []).append(float(e.pow(2).mean().sqrt()) * 2 ** 24)
+    assert all(sum(v) / len(v) < 3 ** -0.5 for v in err.values()), err
+
+
+@pytest.mark.parametrize("size", [1e-12, 3e5, 1e9])
+def test_attn_split_takes_queries_of_any_size(size):
+    """fp32 queries beyond what fp16 holds, up and down, against keys of the inverse size: the scores are ordinary."""
+    D, Hq, Hkv, page, n = 128, 8, 2, 16, 200
+    kc, vc = _fill_cache(16, Hkv, page, D, seed=3)
+    kc = (kc.float() * max(min(1 / size, 1e3), 2e-5)).half()
+    scale = size * float(kc.float().std())
+    qkv = torch.randn(1, (Hq + 2 * Hkv) * D, device=DEV, generator=torch.Generator(DEV).manual_seed(2)) * size
+    qkv[:, Hq * D:] = 0.5
+    ws = (torch.zeros(Hq * 4 * D, device=DEV), torch.zeros(Hq * 8, device=DEV), torch.zeros(Hq, dtype=torch.int32, device=DEV))
+    bt = torch.arange(16, dtype=torch.int32, device=DEV)[None].contiguous()
+    out = ops.attn_decode_rope(qkv, torch.zeros(D // 2, device=DEV), kc, vc, bt, torch.tensor([n], dtype=torch.int32, device=DEV), Hq, Hkv, D, n_splits=4, workspace=ws,
+                               attn_scale=1 / scale)
+    k, v = (c.permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :n].double().repeat_interleave(Hq // Hkv, 0) for c in (kc, vc))
+    q = qkv.double().view(-1, D)[:Hq] * (D ** -0.5 / scale)
+    ref = torch.einsum("hn,hnd->hd", torch.softmax(torch.einsum("hd,hnd->hn", q, k), -1), v)
+    assert nmse(ref.view(1, -1), out) < 2e-7
+
+
 @pytest.mark.parametrize("impl", ["tc", "mma"])
 @pytest.mark.parametrize("D,Hq,Hkv", [(128, 8, 2), (64, 4, 2)])
 @pytest.mark.parametrize("T,pos0,page", [(5, 0, 16), (64, 0, 16), (100, 37, 16), (200, 64, 16), (128, 0, 64), (300, 250, 64), (513, 1000, 64), (1, 400, 8)])
