@@ -73,14 +73,78 @@ __device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_
 //   ROPE: takes the fp32 row of the QKV mat-vec, rotates q in registers, writes the new token's K and V and uses them from shared memory.
 constexpr int ATTN_KEYS_MIN = 128;      // keys a split is worth: 2 tiles per warp, all requested before the dependency wait (700 keys in a
                                         // decode step: as fast as the cluster form; with 256 keys 1.7 us slower)
-struct AttnRange { int eff, begin, end; };
-__device__ __forceinline__ AttnRange attn_range(int len, int n_splits, int split) {
+constexpr int ATTN_KEYS_WHOLE = 320;    // no split up to here: joining costs some 3 us, 64 keys 0.7 (300 keys, 32 heads over 8: 6.5 us whole, 7.2 in three)
+constexpr int ATTN_JOIN_MAX = 40;       // ranges of a query that are worth joining (300 + 8,000 keys, 32 heads over 4, D = 64: 11.9 us with the long one in 22, 12.5 in
+                                        // 30, 14.1 in 46, 16.2 in 63; 300 + 32,000: 19.6 in 31, 20.1 in 47, 21.8 in 73)
+constexpr int ATTN_POOL_NQ = 256;       // (more queries: prompts token by token, not worth a look at every length)
+// Splits of the keys.  One query takes up to n_splits.  Several share a pool (attn_pool): all are cut into ranges of the same length, the
+// shortest that the pool has room for, so that a long sequence among short ones is spread over the machine as it would be alone (32,000 keys
+// beside 31 x 300, 32 heads over 8, D = 128: 44 us; 154 with 16 ranges for every query, 218 with 2).  Places in the pool are those of the ranges' partial results.
+struct AttnRange { int qi, first, eff, begin, end, len; };      // query (-1: no such range), place of its first range, ranges; keys of this one; keys of the query
+__device__ __forceinline__ int attn_per(int len, int n) {         // keys of a range when `len` keys are cut into n: whole tiles
+    return max(16, ((len + n - 1) / n + 15) & ~15);
+}
+__device__ __forceinline__ int attn_pieces(int len, int per) { return len <= max(per, ATTN_KEYS_WHOLE) ? 1 : (len + per - 1) / per; }
+// The range at `place`, or (place < 0) the first one of query `qi`.  All lanes of a warp call it and get the same.
+__device__ __forceinline__ AttnRange attn_range(const AttnParams& p, int place, int qi, int lane) {
     AttnRange r;
-    const int want = min(n_splits, max(1, (len + ATTN_KEYS_MIN - 1) / ATTN_KEYS_MIN));
-    const int per = max(16, ((len + want - 1) / want + 15) & ~15);      // whole tiles
-    r.eff = max(1, (len + per - 1) / per);
-    r.begin = split * per;
-    r.end = min(len, r.begin + per);
+    int per = 0;
+    if (p.pool == 0) {
+        r.qi = place < 0 ? qi : place / p.n_splits;
+        r.first = r.qi * p.n_splits;
+        r.len = p.kv_len[r.qi];
+        per = attn_per(r.len, min(min(p.n_splits, ATTN_JOIN_MAX), max(1, (r.len + ATTN_KEYS_MIN - 1) / ATTN_KEYS_MIN)));
+        r.eff = attn_pieces(r.len, per);
+        if (place >= 0 && place - r.first >= r.eff) r.qi = -1;
+    } else {
+        const int mine = lane < p.nq ? p.kv_len[lane] : 0;
+        auto len_of = [&](int b) { return b == 0 ? mine : b + lane < p.nq ? p.kv_len[b + lane] : 0; };
+        int total = 0, most = 0;
+        for (int b = 0; b < p.nq; b += 32) {
+            total += __reduce_add_sync(0xffffffffu, len_of(b));
+            most = max(most, __reduce_max_sync(0xffffffffu, len_of(b)));
+        }
+        // no query is cut that is about as long as what every slot of the machine has to do anyway
+        const int share = max(ATTN_KEYS_MIN, attn_per(total + total / 5, p.wave));
+        if (most <= max(share, ATTN_KEYS_WHOLE)) {                // every query is a range of its own
+            r.qi = r.first = place < 0 ? qi : place < p.nq ? place : -1;
+            if (r.qi < 0) return r;
+            r.eff = 1;
+            r.len = p.nq <= 32 ? __shfl_sync(0xffffffffu, mine, r.qi) : p.kv_len[r.qi];
+        } else {
+            per = max(share, max(attn_per(total, p.pool - p.nq / 2), attn_per(most, ATTN_JOIN_MAX)));
+            const int enough = attn_per(total, p.pool - p.nq);      // (last ranges are short: at most nq places more than total / per)
+            while (per < enough) {
+                int used = 0;
+                for (int b = 0; b < p.nq; b += 32) used += __reduce_add_sync(0xffffffffu, b + lane < p.nq ? attn_pieces(len_of(b), per) : 0);
+                if (used <= p.pool) break;
+                per = min(enough, (per + (per >> 3) + 15) & ~15);
+            }
+            r.qi = -1;
+            for (int b = 0, at = 0; b < p.nq; b += 32) {
+                const int len = len_of(b), n = b + lane < p.nq ? attn_pieces(len, per) : 0;
+                int upto = n;                                     // ranges of the queries up to this lane's
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int x = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += x;
+                }
+                const unsigned hit = __ballot_sync(0xffffffffu, place < 0 ? b + lane == qi : place >= at + upto - n && place < at + upto);
+                if (hit) {
+                    const int src = __ffs(hit) - 1;
+                    r.qi = b + src;
+                    r.eff = __shfl_sync(0xffffffffu, n, src);
+                    r.first = at + __shfl_sync(0xffffffffu, upto, src) - r.eff;
+                    r.len = __shfl_sync(0xffffffffu, len, src);
+                    break;
+                }
+                at += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (r.qi < 0) return r;
+        }
+    }
+    r.begin = r.eff == 1 || place < 0 ? 0 : (place - r.first) * per;
+    r.end = r.eff == 1 ? r.len : min(r.len, r.begin + per);
     return r;
 }
 struct AttnRope {
@@ -96,10 +160,10 @@ struct AttnRope {
 // One warp joins the partials of `eff` splits of one (query, head): a lane takes D / 32 dims, its loads of 8 splits in flight at a time.
 // (One thread per dim, splits one after the other: 45 us instead of 28.5 for 32,000 keys in 37 splits.)
 template <int D>
-__device__ __forceinline__ void attn_join(const AttnParams& p, size_t head, int eff, int lane) {
+__device__ __forceinline__ void attn_join(const AttnParams& p, int qi, int hq, int first, int eff, int lane) {
     constexpr int E = D / 32;
     constexpr float LOG2E = 1.4426950408889634f;
-    const size_t pi0 = head * p.n_splits;
+    const size_t pi0 = (size_t)hq * p.nq * p.n_splits + first, head = (size_t)qi * p.Hq + hq;
     const float* ml = p.part_ml + pi0 * 2;
     float mn = -INFINITY, ls = 0.f, acc[E];
 #pragma unroll
@@ -142,15 +206,15 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
     extern __shared__ __align__(128) uint8_t as_smem[];
     const int gqa = p.Hq / p.Hkv, R = 8 * NH, groups = (gqa + R - 1) / R;
     const int kvh = blockIdx.y / groups, h0 = (blockIdx.y % groups) * R, G = min(R, gqa - h0), hq0 = kvh * gqa + h0;
-    const int split = blockIdx.x, qi = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     trace_event(p.trace, TR_ATTN | TR_BEGIN);
     // ROPE: length, pages and the cached rows were written at least two launches back (the immediate predecessor is the QKV mat-vec), so
     // the first tiles are requested before the dependency wait.  Otherwise the predecessor wrote the newest K / V row.
     if (!ROPE) pdl_wait();
-    const int len = p.kv_len[qi];
-    const AttnRange rg = attn_range(len, p.n_splits, split);
-    if (split >= rg.eff) return;
-    const int n_old = len - 1;
+    const int place = blockIdx.z * gridDim.x + blockIdx.x;
+    const AttnRange rg = attn_range(p, place, 0, lane);
+    if (rg.qi < 0) return;
+    const int qi = rg.qi, n_old = rg.len - 1;
     const int n_tiles = (rg.end - rg.begin + 15) >> 4, n_mine = n_tiles > warp ? (n_tiles - warp + 3) >> 2 : 0;
     const int* bt = p.block_table + (size_t)(p.bt_row ? p.bt_row[qi] : qi) * p.max_pages;
     uint8_t* ring = as_smem + warp * (STAGES * 2 * TILE);
@@ -433,7 +497,7 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
         if (rg.eff == 1) {
             p.out[((size_t)qi * p.Hq + hq) * D + d] = __float2half_rn(ls > 0.f ? acc / ls : 0.f);
         } else {
-            const size_t pi = ((size_t)qi * p.Hq + hq) * p.n_splits + split;
+            const size_t pi = (size_t)hq * p.nq * p.n_splits + place;
             p.part_o[pi * D + d] = acc;
             if (d == 0) { p.part_ml[pi * 2] = mn; p.part_ml[pi * 2 + 1] = ls; }
         }
@@ -453,7 +517,7 @@ __global__ void __launch_bounds__(128, 2) attn_split_kernel(const AttnParams p, 
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    for (int r = warp; r < G; r += 4) attn_join<D>(p, (size_t)qi * p.Hq + hq0 + r, rg.eff, lane);
+    for (int r = warp; r < G; r += 4) attn_join<D>(p, qi, hq0 + r, rg.first, rg.eff, lane);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -807,18 +871,30 @@ __global__ void attn_combine_kernel(const AttnParams p) {
     const int hq = blockIdx.x, qi = blockIdx.y;
     pdl_wait();
     pdl_launch_dependents();
-    const int eff = attn_range(p.kv_len[qi], p.n_splits, 0).eff;
-    if (eff == 1) return;   // the single split already wrote the final output
-    attn_join<D>(p, (size_t)qi * p.Hq + hq, eff, threadIdx.x);
+    const AttnRange rg = attn_range(p, -1, qi, threadIdx.x);
+    if (rg.eff == 1) return;   // the single range already wrote the final output
+    attn_join<D>(p, qi, hq, rg.first, rg.eff, threadIdx.x);
+}
+
+// Ranges that several queries share: one wave of the kernel's two CTAs an SM, or half a wave more than there are queries - as far as the
+// workspace goes -, so that queries of equal length stay whole where cutting them would only start a second wave (32 x 2,000 keys, 32 heads over 8:
+// 42 us whole, 51 in two each; 16: 26.8 in two, 35 in three; 8: 14.1 in four, 22 in five).  0: every query has its n_splits.
+static void attn_pool(AttnParams& p, int groups) {
+    p.pool = 0;
+    if (p.n_splits <= 1 || p.nq <= 1 || p.nq > ATTN_POOL_NQ) return;
+    p.wave = max(1, 2 * sm_count() / (p.Hkv * groups));
+    p.pool = min(p.nq * p.n_splits, max(p.wave, p.nq + max(1, p.wave / 2)));
 }
 
 template <int D, int NH, bool ROPE>
-static int launch_attn_split(const AttnParams& p, const AttnRope& ra, cudaStream_t s) {
+static int launch_attn_split(AttnParams p, const AttnRope& ra, cudaStream_t s) {
     auto kern = attn_split_kernel<D, NH, ROPE>;
     if (first_use_on_device((const void*)kern))
         DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_split_smem<D>()));
     const int gqa = p.Hq / p.Hkv, groups = (gqa + 8 * NH - 1) / (8 * NH);
-    DLP_CHECK_CUDA(launch_pdl(kern, dim3(p.n_splits, p.Hkv * groups, p.nq), dim3(128), attn_split_smem<D>(), s, p, ra));
+    attn_pool(p, groups);
+    const dim3 grid(p.pool ? p.pool : p.n_splits, p.Hkv * groups, p.pool ? 1 : p.nq);
+    DLP_CHECK_CUDA(launch_pdl(kern, grid, dim3(128), attn_split_smem<D>(), s, p, ra));
     if (p.n_splits > 1 && p.counters == nullptr)
         DLP_CHECK_CUDA(launch_pdl(attn_combine_kernel<D>, dim3(p.Hq, p.nq), dim3(32), 0, s, p));
     return 0;
@@ -1053,9 +1129,8 @@ int attn_prefill(const __half* q, const __half* kc, const __half* vc, const int*
 //   * a launch needs nq * Hq * n_splits * (D + 2) floats and is refused with an error beyond that;
 //   * every call on a device shares the same array, so calls that overlap on the GPU (different streams, or
 //     graphs replayed concurrently) race - serialise them;
-//   * nothing has to start at zero: the partial kernel writes every (query, head, split) slot - empty splits
-//     write m = -inf, l = 0 - before the combine kernel reads it, so stale contents of an earlier call are
-//     never observed.
+//   * nothing has to start at zero: the combine kernel reads the slots of the ranges that the partial kernel had
+//     keys for and wrote, so stale contents of an earlier call are never observed.
 // In host code the array's name is only a handle: the device address is obtained once per device with
 // cudaGetSymbolAddress (device current, return code checked) on the first call there, which therefore must
 // happen outside stream capture.
@@ -1084,8 +1159,8 @@ int attn_paged_static(AttnParams p, int D, cudaStream_t s) {
         dev_ptr[dev] = ptr;
     }
     p.counters = nullptr;                // this entry point keeps the two-kernel combine
-    p.part_o = ptr;                      // [nq, Hq, n_splits, D]
-    p.part_ml = ptr + n_part * (size_t)D;  // [nq, Hq, n_splits, 2]
+    p.part_o = ptr;                      // [Hq, nq * n_splits, D]
+    p.part_ml = ptr + n_part * (size_t)D;  // [Hq, nq * n_splits, 2]
     return attn_paged(p, D, s);
 }
 

@@ -108,10 +108,11 @@ struct AttnParams {
     const int* bt_row;      // [nq] block-table row of each query (nullptr => row = query index)
     const int* kv_len;      // [nq] number of keys visible to each query
     __half* out;            // [nq, Hq, D]
-    float* part_o;          // [nq, Hq, n_splits, D]   (n_splits > 1)
-    float* part_ml;         // [nq, Hq, n_splits, 2]
+    float* part_o;          // [Hq, nq * n_splits, D]   (n_splits > 1)
+    float* part_ml;         // [Hq, nq * n_splits, 2]
     int* counters;          // [nq, Hkv * groups] zero-initialised; non-null => the last split CTA combines in-kernel
     int nq, Hq, Hkv, max_pages, page_size, n_splits;
+    int pool = 0, wave = 0;                // ranges of keys that all queries share (set by the launch; 0: n_splits for each query), ranges that run at once
     unsigned long long* trace = nullptr;   // device timeline buffer, normally null
     int pdl_early = 0;
     int keys_per_split = 64;               // one-launch decode kernel: target keys per cluster member

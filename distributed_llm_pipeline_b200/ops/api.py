@@ -292,17 +292,15 @@ def _attn_cpu(q, k_cache, v_cache, block_table_rows, kv_len, n_head, n_head_kv, 
     return out
 
 
-ATTN_KEYS_MIN = 128      # keys a split is worth (csrc/attention.cu)
+ATTN_KEYS_MIN, ATTN_JOIN_MAX = 128, 40      # keys a split is worth, splits that are worth joining (csrc/attention.cu)
 
 
 def attn_splits(nq: int, n_head_kv: int, group: int, n_sm: int, n_ctx: int) -> int:
-    """Key splits of a decode attention launch (a cap: the kernel takes one per ATTN_KEYS_MIN keys of each query's own length, up to the n_ctx that there can be).  One query: one full
-    wave of the kernel's two CTAs an SM (32,000 keys of 8 KV heads: 28.7 us with 37 splits, 32.1 with 16, 35.1 with 74).  Several: the wave
-    rounded up; their lengths differ, but a split that a short query does not need still has to be started (4 queries of up to 2,000 keys: 9.3 us
-    with 8 splits, 13.5 with 19; 32: 33 us with 2, 36 with 3, 43 with 8; 32 of up to 300: 13 us with 2, 16 with 8)."""
-    pairs = nq * n_head_kv * ((group + 15) // 16)
-    fill = 2 * n_sm // pairs if nq == 1 else (2 * n_sm + pairs - 1) // pairs
-    return max(1, min(fill, (n_ctx + ATTN_KEYS_MIN - 1) // ATTN_KEYS_MIN))
+    """Key splits a query that a decode attention launch needs room for.  One query takes as many as fill the machine once with the kernel's two CTAs an SM (32,000
+    keys of 8 KV heads: 28.7 us with 37 splits, 32.1 with 16, 35.1 with 74).  Several share the room of all of them (attn_pool in csrc/attention.cu)."""
+    wave = max(1, 2 * n_sm // (n_head_kv * ((group + 15) // 16)))
+    room = min(wave, ATTN_JOIN_MAX) if nq == 1 else -(-max(wave, nq + max(1, wave // 2)) // nq)
+    return max(1, min(room, -(-n_ctx // ATTN_KEYS_MIN)))
 
 
 def attn_paged(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,

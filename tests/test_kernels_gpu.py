@@ -483,6 +483,36 @@ def test_attn_split_tiles_and_joins(D, Hq, Hkv, page, n_splits):
     assert int(ws[2].abs().sum()) == 0
 
 
+@pytest.mark.parametrize("lens", [[300] * 31 + [9000], [20, 7000, 330], [321, 320, 0, 1], [2000] * 16, [100 * i for i in range(40)], [5] * 70 + [3000] + [400] * 29, [65] * 290 + [700] * 10])
+@pytest.mark.parametrize("n_splits", [2, 5])
+def test_attn_split_of_uneven_batches(lens, n_splits):
+    """Queries that share a pool of key ranges: one long among short ones, empty ones, more than a warp of queries, more than share (256), pools that are too small
+    for short ranges.  Joined in the kernel and by a second one, against 64 bits; a long one beside short ones takes most of the pool."""
+    D, Hq, Hkv, page, nq = 64, 8, 2, 64, len(lens)
+    need = [(n + page - 1) // page for n in lens]
+    kc, vc = _fill_cache(sum(need) + 1, Hkv, page, D, seed=5)
+    bt = torch.zeros(nq, max(need), dtype=torch.int32)
+    for i, n in enumerate(need):
+        bt[i, :n] = torch.arange(n) + sum(need[:i])
+    bt, kv_len = bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    q = (torch.randn(nq, Hq * D, device=DEV, generator=torch.Generator(DEV).manual_seed(1)) / math.sqrt(D)).half()
+    ws = (torch.full((nq * Hq * n_splits * D,), math.nan, device=DEV), torch.full((nq * Hq * n_splits * 2,), math.nan, device=DEV), torch.zeros(nq * Hq, dtype=torch.int32, device=DEV))
+    out = ops.attn_paged(q, kc, vc, bt, kv_len, Hq, Hkv, D, n_splits=n_splits, workspace=ws)
+    assert torch.equal(out, ops.attn_paged(q, kc, vc, bt, kv_len, Hq, Hkv, D, n_splits=n_splits))
+    assert int(ws[2].abs().sum()) == 0
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert not out[i].any()
+            continue
+        pg = bt[i, :need[i]].long()
+        k, v = (c[pg].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :n].double().repeat_interleave(Hq // Hkv, 0) for c in (kc, vc))
+        ref = (torch.softmax(k @ q[i].view(Hq, D, 1).double(), 1) * v).sum(1).view(-1)
+        assert nmse(ref, out[i]) < 2e-7, (i, n)
+    if lens[-1] == 9000:
+        ranges = int((~ws[1].view(Hq, -1, 2)[0, :, 0].isnan()).sum())
+        assert ranges >= 16
+
+
 @pytest.mark.parametrize("D,Hq,Hkv", [(128, 32, 8), (64, 32, 4), (128, 24, 2)])
 def test_attn_split_arithmetic_is_fp32(D, Hq, Hkv):
     """Sums that cancel show what decode attention rounds: keys with values + 1024, others, and the first keys again with - 1024.  Each rounding of an fp32 sum of
