@@ -84,7 +84,7 @@ class LlamaEngine(EngineCore):
         if last_stage and self.comm.tp_size > 1 and hasattr(self.comm, "reserve_logits") and (v1 - v0) != cfg.vocab_size:
             self.comm.reserve_logits(max_seqs, v1 - v0, f32, dev)     # before any graph is captured
         # splits of the cached keys by batch size (index: queries of the step)
-        n_sm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 0
+        self.n_sm = n_sm = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 0
         self.attn_splits = [0] + [attn_splits if attn_splits is not None else ops.attn_splits(b, self.Hkv, self.Hq // self.Hkv, n_sm, n_ctx) if n_sm else 1
                                   for b in range(1, max_seqs + 1)]
         parts = max(b * ns for b, ns in enumerate(self.attn_splits)) * self.Hq
@@ -102,17 +102,35 @@ class LlamaEngine(EngineCore):
         self.rope_cs = (torch.zeros(max_seqs, self.D // 2, 2, dtype=f32, device=dev)
                         if self.attn_onepass and os.environ.get("DLP_ROPE_TABLE", "1") == "1" else None)
 
-    # attention variants of a decode step of up to 4 sequences: everything in one launch (True) or RoPE + attention (False); larger steps
-    # have the second only
+    # attention variants of a decode step of up to 4 sequences: everything in one launch, with the splits joined through memory (True) or inside a
+    # thread-block cluster ("cluster"), or RoPE + attention (False); larger steps have the last only
     @property
     def _onepass_now(self) -> bool:
         return bool(self._variant)
 
     def _choose_variant(self, B: int, max_len: int):
-        self._variant = self.attn_onepass and B <= 4 and max_len >= self.attn_onepass_min
+        onepass = self.attn_onepass and B <= 4 and max_len >= self.attn_onepass_min
+        lo, hi = self._cluster_range(B)
+        self._variant = "cluster" if onepass and lo < max_len <= hi else onepass
+
+    def _cluster_range(self, B: int) -> tuple[int, int]:
+        """Context lengths (above, up to) at which the cluster form is the faster one: few heads, so that all clusters of 16 blocks run at once, and few products
+        a key (`work`, in fp32 on the CUDA cores).  Against joining through memory, us: 8 heads of 8, D = 128 (work 128): 100 keys 4.3 / 4.2, 300 4.4 / 6.7, 700
+        4.7 / 6.5, 2,000 6.8 / 7.6, 8,000 16 / 12; 32 heads over 4, D = 64 (256): 700 6.2 / 6.6, 2,000 9.3 / 8.2 (a step of tinyllama in
+        Q8_0: 200 keys 689 / 676, 300 684 / 698, two sequences of 500 862 / 911, up to 2,000 944 / 969); 32 over 8, D = 128 (512): 300 8.6 / 7.1."""
+        gqa = self.Hq // self.Hkv
+        group = 4 if gqa % 4 == 0 else 2 if gqa % 2 == 0 else 1
+        work = group * self.D
+        if self.attn_ws is None or work > 256 or self.n_ctx <= work or 16 * B * (self.Hq // group) > 2 * self.n_sm:
+            return 0, 0
+        return work, 2048
 
     def _companion_variants(self) -> list:
-        return [not self._variant] if self.attn_onepass and self.attn_onepass_min > 1 and len(self._active_host) <= 4 else []
+        B = len(self._active_host)
+        if not self.attn_onepass or B > 4:
+            return []
+        reach = [True] + [False] * (self.attn_onepass_min > 1) + ["cluster"] * (self._cluster_range(B)[1] > 0)
+        return [v for v in reach if v != self._variant]
 
     def _graph_ok(self) -> bool:
         moe_lw = next((lw for lw in self.w.layers.values() if lw.router is not None), None)
@@ -442,11 +460,12 @@ class LlamaEngine(EngineCore):
 
     def _attn_decode_onepass(self, il, qkv, T):
         rope_on = self.inv_freq_off is None or self.cfg.layer_uses_rope(il)     # off: no (cos, sin) table, angles from the zero table
+        joined = self.attn_ws is not None and self._variant != "cluster"
         return ops.attn_decode_rope(qkv, self._inv_freq(il), self.kv.k[il], self.kv.v[il], self.kv.block_table, self.kv_len[:T],
-                                    self.Hq, self.Hkv, self.D, bt_row=self.active[:T], n_splits=self.attn_cluster if self.attn_ws is None else self.attn_splits[T],
+                                    self.Hq, self.Hkv, self.D, bt_row=self.active[:T], n_splits=self.attn_splits[T] if joined else self.attn_cluster,
                                     neox=self.cfg.rope_neox, attn_scale=self.attn_scale, out=self.att[:T],
                                     rope_cs=self.rope_cs[:T] if (self.rope_cs is not None and rope_on) else None,
-                                    workspace=self.attn_ws)
+                                    workspace=self.attn_ws if joined else None)
 
     def _attn_prefill_for(self, sid: int, pos0: int):
         def fn(il, q, T):

@@ -199,3 +199,25 @@ def test_block_table_row_is_taken_when_it_is_copied(tmp_models):
     assert eng.seqs[again].pages != first
     eng.kv.free.extend(other)
     assert seen[:3].tolist() == first and table[sid][:3].tolist() == eng.seqs[again].pages
+
+
+def test_decode_attention_changes_its_form_with_the_context(tmp_models):
+    """A sequence that grows past the lengths at which few heads are served by the cluster form: the same logits as from the form with the workspace alone, and all
+    graphs of a batch size are captured at its first step."""
+    logits = []
+    for cluster in (True, False):
+        eng = LlamaEngine(load_weights(tmp_models[("tiny", "F16")], "cuda"), n_ctx=512, max_seqs=2, page_size=16, max_batch_tokens=256)
+        lo, hi = eng._cluster_range(1)
+        assert lo >= 128 and hi > lo and eng._cluster_range(3)[1] >= 0
+        if not cluster:
+            eng._cluster_range = lambda B: (0, 0)
+        sid = eng.alloc_seq()
+        eng.prefill(sid, [3 + i % 50 for i in range(lo - 4)])
+        rows, forms = [], []
+        for t in range(8):
+            rows.append(eng.decode([sid], [5 + t], sample=False)[0].clone())
+            forms.append(eng._variant)
+            assert len(eng._graphs) == (2 if cluster else 1)
+        assert ("cluster" in forms and True in forms) == cluster
+        logits.append(torch.stack(rows))
+    assert nmse(*logits) < 1e-6
