@@ -434,20 +434,23 @@ static int resident_cluster_blocks(Kern kern, unsigned cl, size_t smem, int thre
 
 // How much of an SM's 256 KB is shared memory is left to the driver otherwise, and it keeps what the largest neighbour in the stream asked for:
 // behind attention (196 KB for two blocks) the loads in flight of these kernels - 128 KB of registers to fill an SM - found 28 KB of L1 to return
-// through, and 8 layers of Llama-8B decoded in Q8_0 at 815 us a token instead of 635 (all for shared memory: 1,220; a third: 704).  So half of it is
-// shared memory for one and two tokens, room for two blocks of the widest rows (2 x 52 KB).  Four tokens need more of it and are bound by
-// arithmetic: left to the driver, 1,310 us a step in Q4_K_M against 1,430.
+// through, and 8 layers of Llama-8B decoded in Q8_0 at 815 us a token instead of 635 (all for shared memory: 1,220; a third: 704).  So for one and two
+// tokens half of it is shared memory, or what two blocks take: with half of it 2 x 11,008 columns, 80 KB a block, left one block an SM, and Q8_0
+// took 31 us instead of 21.  Four tokens need more of it and are bound by arithmetic: left to the driver, 1,310 us a step in Q4_K_M against 1,430.
+static int gemv_carveout(int T, size_t smem) {
+    if (T > 2) return -1;
+    const int two = (int)((2 * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));      // (1 KB a block is the system's)
+    return two < 50 ? 50 : two > 100 ? 100 : two;
+}
 template <typename Kern>
-static int gemv_first_use(Kern kern, int T) {
-    if (!first_use_on_device((const void*)kern)) return 0;
-    DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    if (T <= 2) DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 50));
+static int gemv_first_use(Kern kern) {
+    if (first_use_on_device((const void*)kern)) DLP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     return 0;
 }
 
 template <typename Kern>
 static int launch_gemv_v3(Kern kern, const GemvParams& p, int U, size_t x_smem, cudaStream_t stream) {
-    if (int rc = gemv_first_use(kern, p.T)) return rc;
+    if (int rc = gemv_first_use(kern)) return rc;
     const bool dual = p.out_mode == GV_SWIGLU_F16;
     const int rpu = dual ? 1 : 2;
     const int groups = (p.w0.N + rpu - 1) / rpu;
@@ -464,7 +467,7 @@ static int launch_gemv_v3(Kern kern, const GemvParams& p, int U, size_t x_smem, 
     DLP_REQUIRE(((size_t)((groups + blocks - 1) / blocks + 1) * KC * 2 * p.T * sizeof(float)) + ((x_smem + 15) & ~size_t(15)) <= 100 * 1024,
                 "gemv v3: row range too long for shared memory");
     const size_t smem2 = ((x_smem + 15) & ~size_t(15)) + (size_t)((groups + blocks - 1) / blocks + 1) * KC * 2 * p.T * sizeof(float);
-    DLP_CHECK_CUDA(launch_pdl_cluster(kern, dim3(blocks), dim3(256), smem2, stream, cl, p));
+    DLP_CHECK_CUDA(launch_pdl_carveout(kern, dim3(blocks), dim3(256), smem2, stream, cl, gemv_carveout(p.T, smem2), p));
     return 0;
 }
 
@@ -1043,7 +1046,7 @@ __global__ void __launch_bounds__(256, 2) gemv_quant_v3_kernel(const GemvParams 
 
 template <typename Kern>
 static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaStream_t stream, int chunk_w, bool mins) {
-    if (int rc = gemv_first_use(kern, p.T)) return rc;
+    if (int rc = gemv_first_use(kern)) return rc;
     const bool dual = p.out_mode == GV_SWIGLU_F16;
     const int rpu = dual ? 1 : 2;
     const int groups = (p.w0.N + rpu - 1) / rpu;
@@ -1051,15 +1054,16 @@ static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaSt
     if (blocks > groups) blocks = groups;
     const unsigned cl = ar_cluster(p, blocks);
     const int K = p.w0.K, KC = ((K / chunk_w) + 31) >> 5;
-    // (without mins: what the kernel uses and as much again of the sums that it no longer keeps - 2 tokens of 14,336 columns stay with the kernel
-    // below, 25 us against 37 for 4096 x 14336 in Q8_0)
-    const size_t fixed = ((x_smem + 15) & ~size_t(15)) + (size_t)p.T * (K + (K >> 5) * (mins ? 16 : 20));
+    // Two tokens of wide rows in the types without mins: the kernel below, with one pass less over the activations in shared memory (4096 rows of
+    // Q8_0, here / there: 5,632 columns 9.2 / 10.8 us, 8,192 15.6 / 14.8, 11,008 21.1 / 20.0, 14,336 27.2 / 24.1; Q6_K 14,336: 26.4 / 24.6)
+    if (p.T == 2 && !mins && K >= 8192) return -2;
+    const size_t fixed = ((x_smem + 15) & ~size_t(15)) + (size_t)p.T * (K + (K >> 5) * (mins ? 16 : 12));
     blocks = resident_cluster_blocks(kern, cl, fixed + 4096, 256, blocks);
     blocks -= blocks % (int)cl;
     const int max_groups = (groups + blocks - 1) / blocks + 1;
     const size_t smem = fixed + (size_t)max_groups * KC * 2 * p.T * sizeof(float);
     if (smem > 100 * 1024) return -2;   // caller falls back to v1
-    DLP_CHECK_CUDA(launch_pdl_cluster(kern, dim3(blocks), dim3(256), smem, stream, cl, p));
+    DLP_CHECK_CUDA(launch_pdl_carveout(kern, dim3(blocks), dim3(256), smem, stream, cl, gemv_carveout(p.T, smem), p));
     return 0;
 }
 
