@@ -1054,9 +1054,10 @@ static int launch_gemv_qv3(Kern kern, const GemvParams& p, size_t x_smem, cudaSt
     if (blocks > groups) blocks = groups;
     const unsigned cl = ar_cluster(p, blocks);
     const int K = p.w0.K, KC = ((K / chunk_w) + 31) >> 5;
-    // Two tokens of wide rows in the types without mins: the kernel below, with one pass less over the activations in shared memory (4096 rows of
-    // Q8_0, here / there: 5,632 columns 9.2 / 10.8 us, 8,192 15.6 / 14.8, 11,008 21.1 / 20.0, 14,336 27.2 / 24.1; Q6_K 14,336: 26.4 / 24.6)
-    if (p.T == 2 && !mins && K >= 8192) return -2;
+    // Two tokens of wide rows in the types without mins: the kernel below, with one pass less over the activations in shared memory (Q8_0, here / there:
+    // 4096 rows of 5,632 columns 9.2 / 10.8 us, 8,192 15.6 / 14.8 but 3,072 rows of them 13.7 / 14.4, 11,008 21.1 / 20.0, 14,336 27.2 / 24.1; Q6_K 3072 x
+    // 8,192 13.8 / 15.1, 4096 x 11,008 21.0 / 20.4, 14,336 26.4 / 24.6)
+    if (p.T == 2 && !mins && K > 8192) return -2;
     const size_t fixed = ((x_smem + 15) & ~size_t(15)) + (size_t)p.T * (K + (K >> 5) * (mins ? 16 : 12));
     blocks = resident_cluster_blocks(kern, cl, fixed + 4096, 256, blocks);
     blocks -= blocks % (int)cl;
