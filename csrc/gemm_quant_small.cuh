@@ -76,10 +76,18 @@ __device__ __forceinline__ uint32_t fma2_h2(float a, float b, float2 s, float2 o
     const __half2 h = __floats2half2_rn(r.x, r.y);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-__device__ __forceinline__ void unpack4(uint32_t bytes, float half_scale, float off, uint32_t* out) {
-    const float2 s = make_float2(half_scale, half_scale), o = make_float2(off, off);
-    out[0] = fma2_h2(byte_256(bytes, 0), byte_256(bytes, 1), s, o);
-    out[1] = fma2_h2(byte_256(bytes, 2), byte_256(bytes, 3), s, o);
+__device__ __forceinline__ void unpack4(uint32_t bytes, float scale, float off, uint32_t* out, float c = 0.f) {
+    const float2 s = make_float2(scale, scale), o = make_float2(off, off);
+    float f[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { f[k] = byte_256(bytes, k); if (c != 0.f) f[k] += c; }
+    out[0] = fma2_h2(f[0], f[1], s, o);
+    out[1] = fma2_h2(f[2], f[3], s, o);
+}
+// a + b, and whether that is exact (taking the larger one away again leaves exactly the rest; NaN: no)
+__device__ __forceinline__ bool sum_exact(float a, float b, float& s) {
+    s = __fadd_rn(a, b);
+    return __fsub_rn(s, a) == b && __fsub_rn(s, b) == a;
 }
 template <int WT>
 __device__ __forceinline__ void unpack_slice(const uint8_t* st, int r, int j, uint2 d, uint32_t (&out)[32]) {
@@ -137,27 +145,37 @@ __device__ __forceinline__ void unpack_slice(const uint8_t* st, int r, int j, ui
         const uint32_t sc = sc4 >> (16 * (j & 1)), mn = mn4 >> (16 * (j & 1));
         const float s0 = dm.x * fmaf(byte_256(sc, 0), 0.5f, -128.f), s1 = dm.x * fmaf(byte_256(sc, 1), 0.5f, -128.f);
         const float m0 = dm.y * fmaf(byte_256(mn, 0), 0.5f, -128.f), m1 = dm.y * fmaf(byte_256(mn, 1), 0.5f, -128.f);
-        const float o0 = fmaf(-128.f, s0, -m0), o1 = fmaf(-128.f, s1, -m1);
+        // A 4-bit (5-bit) value at the top of the mantissa is 16 (16 + q) (8 (32 + q)): one FMA with scale / 16 and - 16 scale - min gives scale q - min,
+        // rounded once, if that offset is exact in fp32 - as it is unless min and scale are more than some 2^3 or 2^6 apart.  Then q by itself.
+        constexpr float BIAS = WT == W_Q5_K ? 32.f : 16.f, INV = WT == W_Q5_K ? 0.125f : 0.0625f;
+        constexpr int UP = WT == W_Q5_K ? 2 : 3;                  // bits that a value is moved up in its byte
+        float o0, o1;
+        const bool exact0 = sum_exact(-BIAS * s0, -m0, o0), exact1 = sum_exact(-BIAS * s1, -m1, o1);
+        auto all = [&](float c, float p0, float p1) {             // c: what the placed bytes still have to lose
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const uint4 v = *reinterpret_cast<const uint4*>(row + QS + j * 32 + c * 16);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-            uint32_t h[4] = {0u, 0u, 0u, 0u};
-            if constexpr (WT == W_Q5_K) {
-                const uint4 x = *reinterpret_cast<const uint4*>(row + 16 + c * 16);
-                h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t lo = (w[i] & 0x0F0F0F0Fu) | 0x80808080u, hi = ((w[i] >> 4) & 0x0F0F0F0Fu) | 0x80808080u;
+            for (int k = 0; k < 2; ++k) {
+                const uint4 v = *reinterpret_cast<const uint4*>(row + QS + j * 32 + k * 16);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                uint32_t h[4] = {0u, 0u, 0u, 0u};
                 if constexpr (WT == W_Q5_K) {
-                    lo |= ((h[i] >> (2 * j)) & 0x01010101u) << 4;
-                    hi |= ((h[i] >> (2 * j + 1)) & 0x01010101u) << 4;
+                    const uint4 x = *reinterpret_cast<const uint4*>(row + 16 + k * 16);
+                    h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w;
                 }
-                unpack4(lo, 0.5f * s0, o0, out + c * 8 + i * 2);
-                unpack4(hi, 0.5f * s1, o1, out + 16 + c * 8 + i * 2);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    constexpr uint32_t MASK = 0x0F0F0F0Fu << UP;
+                    uint32_t lo = ((w[i] << UP) & MASK) | 0x80808080u, hi = ((w[i] >> (4 - UP)) & MASK) | 0x80808080u;
+                    if constexpr (WT == W_Q5_K) {
+                        lo |= ((h[i] >> (2 * j)) & 0x01010101u) << 6;
+                        hi |= ((h[i] >> (2 * j + 1)) & 0x01010101u) << 6;
+                    }
+                    unpack4(lo, INV * s0, p0, out + k * 8 + i * 2, c);
+                    unpack4(hi, INV * s1, p1, out + 16 + k * 8 + i * 2, c);
+                }
             }
-        }
+        };
+        if (exact0 && exact1) all(0.f, o0, o1);
+        else all(-256.f, -m0, -m1);
     }
 }
 

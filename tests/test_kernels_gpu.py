@@ -208,6 +208,56 @@ def test_residual_sums_repeat(T, N, K, t):
     assert nmse(base.double() + x.double() @ dense.double().T, runs[0]) < 2e-7
 
 
+def _blocks(t, N, K, seed):
+    """Random 4- and 5-bit blocks whose scales and mins lie up to 2^12 apart either way, with zeros and negative ones among them; bytes and 64-bit values."""
+    import numpy as np
+    g = np.random.default_rng(seed)
+    size, n = (144, 8) if t == GGMLType.Q4_K else (176, 8)
+    raw = g.integers(0, 256, (N, K // 256, size), dtype=np.uint8)
+    d, m = (np.float16(g.uniform(0.5, 2, (N, K // 256)) * 2.0 ** g.integers(-13, -1, (N, K // 256)) * g.choice([1, 1, 1, -1, 0], (N, K // 256))) for _ in range(2))
+    raw[..., 0:2], raw[..., 2:4] = d[..., None].view(np.uint8), m[..., None].view(np.uint8)
+    s = raw[..., 4:16].astype(np.int64)
+    scale = np.concatenate([s[..., :4] & 63, (s[..., 8:] & 15) | (s[..., :4] >> 6 << 4)], -1)
+    least = np.concatenate([s[..., 4:8] & 63, (s[..., 8:] >> 4) | (s[..., 4:8] >> 6 << 4)], -1)
+    q = raw[..., -128:].reshape(N, -1, 4, 32)
+    q = np.stack([q & 15, q >> 4], 3).reshape(N, -1, n, 32).astype(np.int64)
+    if t == GGMLType.Q5_K:
+        q += (raw[..., 16:48].reshape(N, -1, 1, 32) >> np.arange(8).reshape(1, 1, 8, 1) & 1) << 4
+    exact = q * (d.astype(np.float64)[..., None] * scale)[..., None] - (m.astype(np.float64)[..., None] * least)[..., None]
+    return DeviceWeight.from_raw(raw.reshape(N, -1), t, (N, K), DEV), torch.from_numpy(exact.reshape(N, K)).to(DEV)
+
+
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q5_K])
+@pytest.mark.parametrize("T", [16, 32, 64])
+def test_few_tokens_see_the_rounded_weights(t, T):
+    """One-hot tokens read the fp16 weights that the tensor cores get: scale q - min in fp32, rounded to fp16 once - also where scale and min are far apart."""
+    N, K = 256, 512
+    w, exact = _blocks(t, N, K, T)
+    want = ops.dequant_rows(w, None, out=torch.empty(N, K, dtype=torch.float16, device=DEV))
+    assert nmse(exact, want) < 1e-7
+    eye = torch.eye(K, device=DEV, dtype=torch.float16)
+    got = torch.cat([ops.linear(w, eye[i:i + T].contiguous(), "f32") for i in range(0, K, T)])
+    assert torch.equal(got, want.float().T)
+
+
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q5_K])
+@pytest.mark.parametrize("T", [1, 2, 4])
+def test_mat_vec_on_mins_is_fp32(t, T):
+    """Activations that 8 bits hold exactly (whole numbers, 127 the largest of 32): what remains is fp32 arithmetic.  Every 32 columns add a product of
+    rounded scale, sum and offset - some 5 roundings of 2^-24 / sqrt(3) of terms as large as |scale q x| + |min x| together, added up at random."""
+    N, K = 512, 4096
+    w, exact = _blocks(t, N, K, 7)
+    g = torch.Generator(DEV).manual_seed(T)
+    x = torch.randint(-126, 127, (T, K), device=DEV, generator=g)
+    x[:, ::32] = 127
+    y = ops.linear(w, x.half(), "f32")
+    ref = x.double() @ exact.T
+    size = (x.double().abs()[:, None] * exact.abs()[None]).view(T, N, -1, 32).sum(-1).pow(2).sum(-1).sqrt()
+    err = float(((y.double() - ref) / size).pow(2).mean().sqrt()) * 2 ** 24
+    print("error / 2^-24:", err)
+    assert err < 5 ** 0.5 / 3 ** 0.5
+
+
 @pytest.mark.parametrize("t", [GGMLType.Q8_0, GGMLType.Q4_K, GGMLType.Q5_K, GGMLType.Q6_K])
 @pytest.mark.parametrize("T,N,K,kib", [(193, 256, 256, 256), (300, 700, 512, 512), (1025, 1280, 768, 1 << 16)])
 def test_linear_quant_prompt_in_pieces(t, T, N, K, kib):
