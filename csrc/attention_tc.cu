@@ -32,8 +32,6 @@ static int launch_fa(const __half* q, const __half* kc, const __half* vc, const 
     return 0;
 }
 
-int attn_prefill_expired(int* out) { return gemm_wait_flag(out); }
-
 int attn_prefill_tc(const __half* q, const __half* kc, const __half* vc, const int* bt_row, __half* out, int T, int pos0, int Hq, int Hkv,
                     int D, int page_size, int n_pages, int max_pages, cudaStream_t s) {
     DLP_REQUIRE(T > 0 && Hq % Hkv == 0 && n_pages > 0 && max_pages > 0, "attn_prefill_tc: bad shape");

@@ -22,6 +22,7 @@
 //   busy; K/V stages form a 2-deep ring.
 #pragma once
 #include <string.h>
+#include "waits.cuh"
 
 #include "kernels.cuh"
 #include "mma.cuh"
@@ -42,20 +43,6 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
         : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// mbarrier wait with a limit: a protocol error ends as an error flag the host reads, not as a GPU that spins forever.  Once the flag is
-// up every later wait gives up at once, so the kernel runs to its end, frees its tensor memory and returns (with wrong results).
-// Without a flag (FA_PAGED) the kernel traps: an error the host sees as well.
-__device__ __forceinline__ void mbar_wait_g(uint64_t* bar, uint32_t parity, int* error) {
-    for (unsigned spins = 0; !mbar_try_wait(bar, parity); ++spins) {
-        if (error != nullptr && (spins & 1023u) == 1023u && *reinterpret_cast<volatile int*>(error) != 0) return;
-        if (spins > (1u << 24)) {
-            if (error == nullptr) __trap();
-            atomicExch(error, 1);
-            return;
-        }
-    }
-}
-
 // MN-major operand in the 128-byte-swizzled layout TMA produces for rows of 64 fp16: atoms of 8 rows (1024 B); `lbo_bytes` =
 // distance between consecutive 64-element chunks along the MN dimension, SBO = 1024 B between groups of 8 rows along K.
 __device__ __forceinline__ uint64_t make_smem_desc_sw128_mn(uint32_t smem_addr, uint32_t lbo_bytes) {
@@ -79,7 +66,6 @@ struct FaParams {
     const float* gate;      // [T, ldg] one logit per query head: the head's output is multiplied by its sigmoid (nullptr: not gated)
     int ldg, V;             // V: value size of a head (<= D2; the rest of the tile is padding)
     float scale;
-    int* error;             // set when a wait ran into its limit
     int window, keep, chunk;       // (FA_PAGED: none) position i sees key j <= i when i - j < window and (chunk > 0) both are in one chunk, or when j < keep
     // FA_TILES
     const int* tile_row0;   // [grid.x] first query row of a tile, and its rows (consecutive positions of one sequence)
@@ -196,14 +182,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     const int pi = min((n0 + pc * ps) / ps, p.max_pages - 1), head = bt_row[pi] * p.Hkv + kvh;
                     return (MODE == FA_TILES && key ? head * p.maps + hq % p.maps : head) * ps;
                 };
-                mbar_wait_g(&k_empty[s], ph ^ 1, p.error);
+                mbar_wait_b(&k_empty[s], ph ^ 1);
                 mbar_expect_tx(&k_full[s], Cfg::K_BYTES);
                 for (int pc = 0; pc < chunks; ++pc) {
                     const int row = row_of(pc, true);
                     for (int kb = 0; kb < KB; ++kb)
                         tma_load_2d(sm_k + s * Cfg::K_BYTES + kb * (BN * 128) + pc * (ps * 128), &tm_k, &k_full[s], (MODE == FA_ROWS ? kvh * D1 : 0) + kb * 64, row);
                 }
-                mbar_wait_g(&v_empty[s], ph ^ 1, p.error);
+                mbar_wait_b(&v_empty[s], ph ^ 1);
                 mbar_expect_tx(&v_full[s], Cfg::V_BYTES);
                 for (int pc = 0; pc < chunks; ++pc) {
                     const int row = row_of(pc, false);
@@ -219,10 +205,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             constexpr uint32_t idesc_o = make_idesc_f16_bmn(BM, D2, FMT);
             auto issue_pv = [&](int j) {
                 const int s = j & 1;
-                mbar_wait_g(&v_full[s], (uint32_t)(j >> 1) & 1u, p.error);
+                mbar_wait_b(&v_full[s], (uint32_t)(j >> 1) & 1u);
 #pragma unroll
                 for (int h = 0; h < HALVES; ++h) {
-                    mbar_wait_g(&p_full[h], (uint32_t)j & 1u, p.error);
+                    mbar_wait_b(&p_full[h], (uint32_t)j & 1u);
                     tc_fence_after();
 #pragma unroll
                     for (int kk = h * (BN / 16 / HALVES); kk < (h + 1) * (BN / 16 / HALVES); ++kk) {
@@ -237,12 +223,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 }
                 tc_commit(&v_empty[s]);
             };
-            mbar_wait_g(q_full, 0, p.error);
+            mbar_wait_b(q_full, 0);
             for (int i = 0; i < n_tiles; ++i) {
                 const int s = i & 1;
                 const uint32_t ph = (uint32_t)(i >> 1) & 1u;
-                mbar_wait_g(&k_full[s], ph, p.error);
-                mbar_wait_g(&s_free[s], ph ^ 1, p.error);
+                mbar_wait_b(&k_full[s], ph);
+                mbar_wait_b(&s_free[s], ph ^ 1);
                 tc_fence_after();
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) {
@@ -276,7 +262,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         for (int i = 0; i < n_tiles; ++i) {
             const int s = i & 1;
             const int n0 = key_of(i) + half * CW;
-            mbar_wait_g(&s_full[s], (uint32_t)(i >> 1) & 1u, p.error);
+            mbar_wait_b(&s_full[s], (uint32_t)(i >> 1) & 1u);
             tc_fence_after();
             uint32_t sv[CW];
 #pragma unroll
@@ -321,7 +307,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             l_run = l_run * alpha + (sum[0] + sum[1]);
             m_run = m_new;
             if (i > 0) {
-                mbar_wait_g(&pv_done[half], (uint32_t)(i - 1) & 1u, p.error);       // P.V of the previous tile has read P and updated O
+                mbar_wait_b(&pv_done[half], (uint32_t)(i - 1) & 1u);       // P.V of the previous tile has read P and updated O
                 tc_fence_after();
                 if (__any_sync(0xffffffffu, alpha != 1.f)) {      // a row maximum grew: rescale this warp's 32 rows of O
 #pragma unroll 1
@@ -359,7 +345,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             if (lane == 0) mbar_arrive(&p_full[half]);
         }
         // epilogue: O / l in the output type; with two halves their accumulators are joined here
-        for (int h = 0; h < HALVES; ++h) mbar_wait_g(&pv_done[h], (uint32_t)(n_tiles - 1) & 1u, p.error);
+        for (int h = 0; h < HALVES; ++h) mbar_wait_b(&pv_done[h], (uint32_t)(n_tiles - 1) & 1u);
         tc_fence_after();
         float w0 = 1.f, w1 = 0.f;
         if constexpr (HALVES == 2) {
@@ -438,8 +424,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             __syncwarp();
         }
     }
-    if (p.error != nullptr && threadIdx.x == 0 && *reinterpret_cast<volatile int*>(p.error) != 0)
-        for (int i = 0; i < 1000; ++i) __nanosleep(1000);      // a wait gave up: copies in flight land before the block goes away
+    gemm_wait_aftermath();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

@@ -11,7 +11,7 @@ FLAGS=(-gencode arch=compute_100a,code=sm_100a -O3 -lineinfo -std=c++17 -Xcompil
 case "$PART" in
   all) OBJ="$HERE/build"; LIB="$OUT/libdlp_b200.so"; SRC=("$HERE"/*.cu) ;;
   layers) OBJ="$HERE/build/layers"; LIB="$OUT/libdlp_b200_layers.so"; FLAGS+=(-DDLP_LAYERS_ONLY)
-          SRC=("$HERE"/layers_*.cu "$HERE"/capi_layers.cu "$HERE"/capi_core.cu "$HERE"/elementwise.cu "$HERE"/gemm_tcgen05.cu "$HERE"/gemm_pair.cu "$HERE"/moe.cu) ;;
+          SRC=("$HERE"/layers_*.cu "$HERE"/capi_layers.cu "$HERE"/capi_core.cu "$HERE"/elementwise.cu "$HERE"/gemm_tcgen05.cu "$HERE"/gemm_pair.cu "$HERE"/moe.cu "$HERE"/waits.cu) ;;
   *) echo "build.sh: unknown part '$PART'" >&2; exit 2 ;;
 esac
 mkdir -p "$OBJ" "$OUT"

@@ -134,15 +134,6 @@ int dlp_rs_norm_ag(const dlp_rs_norm_ag_desc* d, void* stream) {
     return rs_norm_ag(a, (cudaStream_t)stream);
 }
 
-int dlp_gemm_wait_expired(int* out) {
-    DLP_REQUIRE(out, "dlp_gemm_wait_expired: null argument");
-    *out = 0;
-    int rc = gemm_pair_expired(out);
-    if (!rc) rc = gemm_quant_small_expired(out);
-    if (!rc) rc = gemv_expired(out);
-    return rc ? rc : attn_prefill_expired(out);
-}
-
 static int linear_impl(const dlp_weight* w0, const dlp_weight* w1, const void* x, const float* norm_w, float eps, void* y,
                        int ldy, int out_mode, int T, void* scratch, size_t scratch_bytes, void* ws, size_t ws_bytes, void* stream) {
     DLP_REQUIRE(w0 && w0->base && x && y, "dlp_linear: null argument");

@@ -124,6 +124,6 @@ int dlp_layers_gqa_flash(const dlp_gqa_args* a, void* stream) {
     DLP_REQUIRE(a, "dlp_layers_gqa_flash: null argument");
     return gqa_flash(*reinterpret_cast<const GqaArgs*>(a), (cudaStream_t)stream);
 }
-int dlp_layers_rows_attention_error(int* flag) { return rows_attention_error(flag); }
+int dlp_layers_rows_attention_error(int* flag) { return dlp_wait_status(flag); }
 
 }  // extern "C"

@@ -29,8 +29,6 @@ static PairPlan pair_plan(int T, int N, int K, int na, bool split, const GemmGro
     return best;
 }
 
-int gemm_pair_expired(int* out) { return gemm_wait_flag(out); }
-
 template <int NA, int AB_FMT>
 static int launch_pair(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const GemmParams& p, const PairPlan& pl, cudaStream_t stream) {
     auto kern = gemm_pair_kernel<NA, AB_FMT>;

@@ -30,6 +30,4 @@ int gemm_quant_small(const QWeight& w0, const QWeight& w1, int na, int wtype, in
     DLP_REQUIRE(false, "gemm_quant: unsupported weight type %d or token tile %d", wtype, bt);
 }
 
-int gemm_quant_small_expired(int* out) { return gemm_wait_flag(out); }
-
 }  // namespace dlp

@@ -266,6 +266,7 @@ gemm_quant_small_kernel(const __grid_constant__ QsMaps tw0, const __grid_constan
             constexpr uint32_t idesc = make_idesc_f16(GEMM_BM, BT, 0);
             int s = 0, as = 0;
             uint32_t ph = 0, aph = 0;
+            if (!grouped) pdl_wait();                               // (X comes after that; the limit of the waits counts from there)
             for (int u = 0; u < units; ++u) {
                 mbar_wait_b(&raw_full[s], ph);
                 const uint32_t xs = smem_u32(smem + s * Cfg::STAGE + NA * Fmt::RAW);
@@ -303,6 +304,7 @@ gemm_quant_small_kernel(const __grid_constant__ QsMaps tw0, const __grid_constan
         const int group = (warp - 2) >> 2;                      // every other slice
         int s = 0, as = group;
         uint32_t ph = 0, aph = 0;
+        if (!grouped) pdl_wait();                                   // (as above; the epilogue reads and writes what a predecessor may still use)
         for (int u = 0; u < units; ++u) {
             const uint2 e0 = scales(qw0, u + 1), e1 = NA == 2 ? scales(qw1, u + 1) : d1;      // (a unit ahead)
             mbar_wait_b(&raw_full[s], ph);
@@ -329,7 +331,6 @@ gemm_quant_small_kernel(const __grid_constant__ QsMaps tw0, const __grid_constan
             d0 = e0;
             d1 = e1;
         }
-        if (!grouped) pdl_wait();                               // the epilogue reads and writes what a predecessor may still use
         pdl_launch_dependents();
         if (group == 0) {
             mbar_wait_b(done, 0);

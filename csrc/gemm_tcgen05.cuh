@@ -171,7 +171,7 @@ __device__ __forceinline__ void gemm_drain(const GemmParams& p, uint32_t tmem_ba
     const int n = n_out0 + n_local;
     const float bias = p.epilogue == EPI_TAIL_BF16 && p.tail.bias != nullptr && n < p.N ? p.tail.bias[n] : 0.f;      // (requested before the accumulators are there)
     if (any) {
-        mbar_wait(tmem_full_bar, 0);
+        mbar_wait_b(tmem_full_bar, 0);
         tc_fence_after();
     }
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -365,7 +365,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             int stage = 0;
             uint32_t phase = 0;
             for (int kb = first; kb < num_kb; ++kb) {
-                mbar_wait(&empty_bar[stage], phase);
+                mbar_wait_b(&empty_bar[stage], phase);
                 load_w(kb, stage);
                 tma_load_2d(smem_b + stage * Cfg::B_BYTES, &tm_x, &full_bar[stage], (kb_begin + kb) * GEMM_BK, t0);
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -377,8 +377,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             constexpr uint32_t idesc = make_idesc_f16(GEMM_BM, BT, AB_FMT);
             int stage = 0;
             uint32_t phase = 0;
+            if (ahead) pdl_wait();                                 // (the tokens come after that; the limit of the wait counts from there)
             for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait(&full_bar[stage], phase);
+                mbar_wait_b(&full_bar[stage], phase);
                 tc_fence_after();
                 const uint64_t da0 = make_smem_desc_sw128(smem_u32(smem_a0 + stage * Cfg::A_BYTES));
                 const uint64_t da1 = make_smem_desc_sw128(smem_u32(smem_a1 + stage * Cfg::A_BYTES));
@@ -405,7 +406,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                 const int kc = (kb_begin + kb) * GEMM_BK;
                 prefetch_row_slice<WT>(qw0, n0 + r, kc + 4 * GEMM_BK);
                 if (NA == 2) prefetch_row_slice<WT>(qw1, n0 + r, kc + 4 * GEMM_BK);
-                mbar_wait(&empty_bar[stage], phase ^ 1);
+                if (ahead && kb == STAGES) pdl_wait();             // (from here on the MMAs, which need the tokens, are waited for)
+                mbar_wait_b(&empty_bar[stage], phase ^ 1);
                 dequant_row_slice<WT>(qw0, n0 + r, kc, smem_a0 + stage * Cfg::A_BYTES, r);
                 if (NA == 2) dequant_row_slice<WT>(qw1, n0 + r, kc, smem_a1 + stage * Cfg::A_BYTES, r);
                 fence_proxy_async();   // generic-proxy smem writes -> visible to tcgen05 (async proxy)
@@ -418,6 +420,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         pdl_launch_dependents();
         gemm_drain<BT, NA, AB_FMT>(p, tmem_base, tmem_full_bar, num_kb > 0, n_out0, t0, t_end);
     }
+    gemm_wait_aftermath();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

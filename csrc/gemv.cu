@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(288, 1) gemv_bulk_kernel(const GemvParams p, c
         // ===== producer: refill ring slots as the consumers release them =====
         if (lane == 0) {
             for (int it = S; it < n_local; ++it) {
-                mbar_wait(&empty[it % S], ((it / S) - 1) & 1);
+                mbar_wait_b(&empty[it % S], ((it / S) - 1) & 1);
                 issue(it);
             }
         }
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(288, 1) gemv_bulk_kernel(const GemvParams p, c
         const int kspan = K / wpr, k_begin = sub * kspan;
         for (int it = 0; it < n_local; ++it) {
             const int s = it % S;
-            mbar_wait(&full[s], (it / S) & 1);
+            mbar_wait_b(&full[s], (it / S) & 1);
             const uint8_t* st = ring + (size_t)s * stage_bytes;
             const uint8_t* w0r = st + (size_t)r * row_bytes;
             const uint8_t* w1r = st + (size_t)(R + r) * row_bytes;
@@ -1255,8 +1255,6 @@ static int launch_gemv_q6_ring(const GemvParams& p, cudaStream_t stream) {
     }
     return -2;
 }
-
-int gemv_expired(int* out) { return gemm_wait_flag(out); }
 
 // ---- MoE router: softmax over all experts -> top-k -> renormalise (llama-graph.cpp:1039-1139; topk-moe.cu) ---------------
 __global__ void moe_route_kernel(const float* __restrict__ logits, int n_expert, int top_k, int* __restrict__ ids, float* __restrict__ w) {

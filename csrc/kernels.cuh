@@ -155,11 +155,6 @@ int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, i
 // the same for prompts: pieces of the weights unpacked to `scratch` (at least 256 rows of fp16, twice with w1), each multiplied by gemm_f16
 int gemm_quant_pieces(const QWeight& w0, const QWeight* w1, int wtype, const void* x, void* y, int ldy, int T, int epilogue, void* scratch,
                       size_t scratch_bytes, cudaStream_t stream);
-// *out |= 1 when a bounded wait of the named kernels has run out on the current device since the library was loaded
-int gemm_pair_expired(int* out);
-int gemm_quant_small_expired(int* out);
-int gemv_expired(int* out);
-int attn_prefill_expired(int* out);
 // MoE routing plan + data movement around the grouped GEMMs (moe.cu)
 int moe_route_ex(const float* logits, int ld, int T, int n_expert, int top_k, int renorm, int* ids, float* w, cudaStream_t s);
 int moe_plan(const int* ids, int n_assign, int n_expert, int bt, int* pos, int* src, int* bounds, int* tile_expert, int* tile_row0,

@@ -359,8 +359,6 @@ int latent_gather(const void* cache, const int* bt, int page, int Rc, void* out,
 int head_rows(const float* x, int ldx, int D, int Dp, int H, void* out, int T, cudaStream_t s);
 int rows_attention(const void* q, const void* kv, int ldkv, int S, int T, int pos0, int H, int Dp, int Vp, int V, int window, float scale, const float* gate, int ldg, void* out,
                    int ldo, cudaStream_t s);
-int rows_attention_error(int* flag);
-int* flash_error_flag();      // device flag a bounded wait raises (nullptr: error set)
 
 
 // Grouped-query softmax attention over paged keys [pages, G * maps, page, Dc] and values [pages, G, page, Vc]: position i sees key j <= i

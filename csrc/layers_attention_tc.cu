@@ -5,15 +5,6 @@
 
 namespace dlp {
 
-__device__ int g_rows_error;     // a wait of the flash kernel ran into its limit since the library was loaded
-
-int* flash_error_flag() {
-    int* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress((void**)&p, g_rows_error);
-    if (e != cudaSuccess) set_error("flash_error_flag: %s", cudaGetErrorString(e));
-    return e == cudaSuccess ? p : nullptr;
-}
-
 // latent rows 0 .. S-1 of one request, out of its pages
 __global__ void __launch_bounds__(128) latent_gather_kernel(const uint4* cache, const int* bt, int page, int chunks, uint4* out) {
     pdl_wait();
@@ -67,7 +58,6 @@ int rows_attention(const void* q, const void* kv, int ldkv, int S, int T, int po
     FaParams p;
     memset(&p, 0, sizeof(p));
     p.out = out; p.T = T; p.pos0 = pos0; p.Hq = H; p.Hkv = H; p.page_size = 128; p.max_pages = 1; p.ldo = ldo; p.gate = gate; p.ldg = ldg; p.V = V; p.scale = scale; p.window = window;
-    if ((p.error = flash_error_flag()) == nullptr) return -1;
     const void* v = (const uint8_t*)kv + (size_t)H * Dp * 2;
     if (Dp == 64 && Vp == 64) return launch_rows<64, 64>(q, kv, v, ldkv, S, p, s);
     if (Dp == 64 && Vp == 128) return launch_rows<64, 128>(q, kv, v, ldkv, S, p, s);
@@ -77,14 +67,4 @@ int rows_attention(const void* q, const void* kv, int ldkv, int S, int T, int po
     if (Dp == 192 && Vp == 128) return launch_rows<192, 128>(q, kv, v, ldkv, S, p, s);
     DLP_REQUIRE(false, "rows_attention: head sizes %d / %d", Dp, Vp);
 }
-// 0, or 1 when a wait of a flash kernel gave up since the last call (synchronises)
-int rows_attention_error(int* flag) {
-    DLP_CHECK_CUDA(cudaMemcpyFromSymbol(flag, g_rows_error, sizeof(int)));
-    if (*flag) {
-        const int zero = 0;
-        DLP_CHECK_CUDA(cudaMemcpyToSymbol(g_rows_error, &zero, sizeof(int)));
-    }
-    return 0;
-}
-
 }  // namespace dlp

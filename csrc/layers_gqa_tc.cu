@@ -33,7 +33,6 @@ int gqa_flash(const GqaArgs& a, cudaStream_t s) {
     p.out = a.out; p.T = a.T; p.Hq = a.H; p.Hkv = a.G; p.page_size = a.page_size; p.max_pages = a.max_pages; p.ldo = a.ldo; p.V = a.V; p.scale = a.scale;
     p.q_head = a.Dc; p.tile_row0 = a.tile_row0; p.tile_rows = a.tile_rows; p.pos = a.pos; p.tok_slot = a.tok_slot; p.block_table = a.block_table; p.window = a.window; p.keep = a.keep;
     p.chunk = a.chunk; p.maps = a.maps; p.out_f32 = a.maps > 1;
-    if ((p.error = flash_error_flag()) == nullptr) return -1;
     if (a.Dc <= 64) return a.Vc <= 64 ? launch_tiles<64, 64>(a, p, s) : launch_tiles<64, 128>(a, p, s);
     return a.Vc <= 64 ? launch_tiles<128, 64>(a, p, s) : launch_tiles<128, 128>(a, p, s);
 }

@@ -12,6 +12,7 @@ from dataclasses import dataclass, field
 import torch
 
 from ..ops import api as ops
+from ..ops import lib as _lib
 
 
 @dataclass
@@ -142,6 +143,9 @@ class EngineCore:
         self.max_tokens = max(max_batch_tokens, max_seqs)
         self.max_rows = M = self.max_tokens + 8   # head-room: the sequence-parallel path pads T up to a multiple of tp
         self.rstate = RecurrentState({}, max_seqs, dev)
+        if torch.device(dev).type == "cuda":
+            with torch.cuda.device(dev):
+                _lib.watch_waits(torch.cuda.current_device())
         self.seqs: dict[int, Sequence] = {}
         self._free_sids = list(range(max_seqs - 1, -1, -1))
         i32 = torch.int32
@@ -287,7 +291,9 @@ class EngineCore:
                use_graph: bool = True):
         """One token for each sequence in `sids` (any subset of slots; batch row i belongs to sids[i]).
         tokens: host ints / tensor, or None to feed back the previously sampled tokens (device resident).
-        Returns next-token ids (device int32 [B]) when sampling, else logits [B, vocab]; or hidden states."""
+        Returns next-token ids (device int32 [B]) when sampling, else logits [B, vocab]; or hidden states.  Raises DlpError when a wait inside an earlier
+        call's kernels ran out (_lib.check_waits: for callers that have read a result, to ask at once)."""
+        _lib.check_waits()
         B = len(sids)
         for sid in sids:
             seq = self.seqs[sid]
@@ -387,11 +393,13 @@ class EngineCore:
                                  torch.empty(1, dtype=torch.int32, device=self.device))
         self.next_tok[:1].copy_(tok)
         out = [int(tok[0])]
+        _lib.check_waits()
         for _ in range(n_predict - 1):
             if out[-1] in stop_ids:
                 break
             nt = self.decode([sid])
             out.append(int(nt[0]))
+            _lib.check_waits()
         if own:
             self.free_seq(sid)
         return out

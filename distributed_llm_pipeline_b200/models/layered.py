@@ -180,9 +180,9 @@ class LayeredEngine(EngineCore):
         if comm is not None and comm.tp_size > 1 or not (first_stage and last_stage):
             raise NotImplementedError(f"{cfg.arch}: layer-list models run on one GPU (no tensor-parallel or pipeline split)")
         dev = weights.tok_embd.device
-        self._init_core(weights, n_ctx, max_seqs, page_size, max_batch_tokens, comm, True, True, dev)
         if dev.type == "cuda":
             lops.load_library()
+        self._init_core(weights, n_ctx, max_seqs, page_size, max_batch_tokens, comm, True, True, dev)
         self.dtype = weights.tok_embd.planes[0].dtype
         self.E = cfg.n_embd
         self.runs = cfg.layer_runs()

@@ -17,6 +17,7 @@ import os
 import torch
 
 from ..ops import api as ops
+from ..ops import lib as _lib
 from .engine import EngineCore, NullComm, PagedKVCache, Sequence  # noqa: F401 (Sequence, NullComm: part of this module's surface)
 from .reference import limit_to_groups, rope_attn_scale, rope_inv_freq
 from .weights import ModelWeights
@@ -619,6 +620,7 @@ class LlamaEngine(EngineCore):
         """Append `tokens` to sequence `sid`.  Returns logits [vocab] of the last token (last stage) or the
         hidden states [T, E] to hand to the next pipeline stage.  `all_logits=True` (single chunk, tp == 1 or the
         NCCL TP path) returns logits [T, vocab] for every appended token (speculative verification, perplexity)."""
+        _lib.check_waits()
         seq = self.seqs[sid]
         tokens = torch.as_tensor(tokens, dtype=torch.int32)
         n = tokens.numel()

@@ -490,8 +490,8 @@ def gqa_flash(m, q, kc, vc, block_table, tok_slot, pos, tiles, out, T: int):
 
 
 def check_waits():
-    """Raise if a wait inside an attention kernel gave up since the last call (synchronises the device)."""
+    """Raise if a wait inside a kernel gave up since the last call (synchronises the device)."""
     flag = C.c_int(0)
-    _lib.check(_lib.load().dlp_layers_rows_attention_error(C.byref(flag)), "rows_attention_error")
+    _lib.check(_lib.load().dlp_wait_status(C.byref(flag)), "wait_status")
     if flag.value:
-        raise _lib.DlpError("a wait inside the attention kernel ran into its limit")
+        raise _lib.WaitError("a wait inside a kernel ran into its limit: the results since the last check are not valid")

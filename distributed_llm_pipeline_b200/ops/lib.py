@@ -97,6 +97,11 @@ def _declare(lib):
         "dlp_layers_gqa_attention": (i32, [vp, i32, i32, vp]),
         "dlp_layers_gqa_flash": (i32, [vp, vp]),
         "dlp_layers_rows_attention_error": (i32, [vp]),
+        "dlp_wait_watch": (i32, [vp]),
+        "dlp_wait_status": (i32, [vp]),
+        "dlp_gemm_wait_expired": (i32, [vp]),
+        "dlp_set_wait_limit": (i32, [C.c_double]),
+        "dlp_wait_probe": (i32, [vp]),
         "dlp_gemv_moe": (i32, [W, W, vp, vp, f32, vp, i32, i32, vp, i32, vp, vp]),
     }
     for name, (res, args) in sigs.items():
@@ -150,6 +155,37 @@ def load_layers():
 
 class DlpError(RuntimeError):
     pass
+
+
+class WaitError(DlpError):
+    """A wait inside a kernel ran into its limit: what was computed since the last check is not valid."""
+
+
+_wait_words: dict[int, C.c_int32] = {}      # by library: not 0 when a wait inside one of its kernels ran out
+_watched: set[tuple[int, int]] = set()
+
+
+def watch_waits(device: int):
+    """Have the kernels on `device` (the current one) report waits that run out, for check_waits.  Outside of captures."""
+    lib = load()
+    if (lib._handle, device) in _watched:
+        return
+    word = C.c_void_p()
+    check(lib.dlp_wait_watch(C.byref(word)), "wait_watch")
+    _wait_words[lib._handle] = C.c_int32.from_address(word.value)
+    _watched.add((lib._handle, device))
+
+
+def check_waits():
+    """Raise if a wait inside a kernel ran out since the last check, as far as the device has got (a load from host memory).  What was computed since then is
+    not to be trusted; the status is cleared, so that the kernels wait again."""
+    for word in _wait_words.values():
+        if word.value:
+            flag = C.c_int(0)
+            for lib in (_lib, _lib_layers):
+                if lib is not None and lib._handle in _wait_words:
+                    check(lib.dlp_wait_status(C.byref(flag)), "wait_status")
+            raise WaitError("a wait inside a kernel ran into its limit: the results since the last check are not valid")
 
 
 def check(rc: int, what: str = ""):

@@ -20,6 +20,7 @@ from typing import Callable
 
 import torch
 
+from ..ops.lib import WaitError, check_waits
 from ..utils.tokenizer import StreamDecoder, Tokenizer
 from .sampler import Sampler, SamplingParams
 
@@ -349,6 +350,7 @@ class Scheduler:
                     else:
                         logits = self.eng.decode(sids, toks, sample=False)
                         new = self._sample_rows(logits, gen)
+                    check_waits()
                 except RuntimeError as e:
                     for s in gen:
                         self._fail(s, str(e))
@@ -453,6 +455,10 @@ class Scheduler:
         block = [s.next_token] + draft
         try:
             pred = self.eng.prefill(s.sid, block, all_logits=True).argmax(-1).tolist()
+            check_waits()
+        except WaitError as e:
+            self._fail(s, str(e))
+            return True
         except (RuntimeError, NotImplementedError):
             return False
         n_ok = 0

@@ -119,9 +119,16 @@ int dlp_swiglu(const void* gate_up, int is_f16, void* out_f16, int T, int F, int
 int dlp_advance(int32_t* seq_len, const int32_t* active, int32_t* pos, int32_t* slot, int32_t* kv_len,
                 const int32_t* block_table, int max_pages, int page_size, int n, void* stream);
 
-/* *out = 1 when a wait inside one of the tensor-core kernels has run into its limit on the current device since the library was loaded (it then
- * returned with wrong results instead of spinning on), else 0.  Synchronises with the device. */
+/* Waits inside kernels are bounded: one that lasts longer than the limit raises a status, and its kernel, and those behind it, return with wrong
+ * results instead of spinning on.  dlp_wait_watch gives a word in host memory that is then not 0 (for the current device from this call on, outside of
+ * stream captures; read it behind any synchronisation, at the cost of a load).  dlp_wait_status: *out = 1 when a wait ran out since the last call, or 0;
+ * synchronises with the device and clears the status, so that later launches wait again.  dlp_gemm_wait_expired: the same without clearing.
+ * dlp_set_wait_limit: seconds (2 at the start), for the current device.  dlp_wait_probe launches a kernel whose one wait runs out, to try it. */
+int dlp_wait_watch(const volatile int32_t** word);
+int dlp_wait_status(int* out);
 int dlp_gemm_wait_expired(int* out);
+int dlp_set_wait_limit(double seconds);
+int dlp_wait_probe(void* stream);
 
 /* Paged attention for nq queries (decode, batched decode, or one query per prefill token).
  * q/out fp16 [nq,Hq,D]; kv_len[q] keys visible; bt_row[q] selects the block-table row (NULL: q).

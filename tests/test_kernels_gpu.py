@@ -2,6 +2,7 @@
 
 Metric and thresholds follow the reference's op tests (NMSE; MUL_MAT / FLASH_ATTN_EXT 5e-4:
 llama.cpp/tests/test-backend-ops.cpp:273-287,3716-3718,6049-6051)."""
+import ctypes
 import math
 
 import pytest
@@ -1010,3 +1011,38 @@ def test_rope_rows_of_a_prompt():
                 ops.rope_kv(qkv[i:i + 5], pos[i:i + 5], slot[i:i + 5], inv, want[1], want[2], Hq, Hkv, D, neox, q_out=want[0][i:i + 5])
             for a, b in zip(got, want):
                 assert nmse(b, a) < 1e-8, (D, n_rot, neox)
+
+
+def test_a_wait_that_runs_out_is_an_error_once(tmp_models):
+    """A wait that nothing ends returns after its limit and raises the status: the engine's next call fails, the one after it works, and the kernels wait again.  The
+    status is also there for callers that ask for it with a synchronisation."""
+    from distributed_llm_pipeline_b200.models.llama import LlamaEngine
+    from distributed_llm_pipeline_b200.models.weights import load_weights
+    from distributed_llm_pipeline_b200.ops import layers as lops
+    from distributed_llm_pipeline_b200.ops import lib as L
+    lib, flag = L.load(), ctypes.c_int(0)
+    eng = LlamaEngine(load_weights(tmp_models[("tiny", "F16")], "cuda"), n_ctx=256, max_seqs=1, page_size=16, max_batch_tokens=64)
+    L.check_waits()
+    L.check(lib.dlp_set_wait_limit(0.02), "set_wait_limit")
+    try:
+        sid = eng.alloc_seq()
+        want = eng.prefill(sid, list(range(1, 20))).clone()
+        for again in (lambda: eng.prefill(sid, [5]), lambda: eng.decode([sid], [5], sample=False)):
+            L.check(lib.dlp_wait_probe(None), "wait_probe")
+            torch.cuda.synchronize()
+            L.check(lib.dlp_gemm_wait_expired(ctypes.byref(flag)), "wait_expired")
+            assert flag.value == 1
+            with pytest.raises(L.WaitError):
+                again()
+            L.check(lib.dlp_gemm_wait_expired(ctypes.byref(flag)), "wait_expired")
+            assert flag.value == 0
+            eng.truncate_seq(sid, 0)
+            assert torch.equal(eng.prefill(sid, list(range(1, 20))), want)
+            again()
+        L.check(lib.dlp_wait_probe(None), "wait_probe")
+        with pytest.raises(L.WaitError):
+            lops.check_waits()
+        lops.check_waits()
+    finally:
+        L.check(lib.dlp_set_wait_limit(2.0), "set_wait_limit")
+    assert lib.dlp_set_wait_limit(0.0) != 0
