@@ -384,9 +384,12 @@ int rope_kv(const void* qkv, int qkv_is_f16, const int* pos, const int* slot, co
     DLP_REQUIRE((qn == nullptr) == (kn == nullptr), "rope_kv: q/k norm weights come as a pair");
     const bool ex = bias != nullptr || qn != nullptr;
     if (qn != nullptr) DLP_REQUIRE(256 % (D / 2) == 0 && (D / 2 >= 32 || (D / 2 & (D / 2 - 1)) == 0), "rope_kv: qk-norm needs D/2 | 256 (D=%d)", D);
-    // from 64 tokens on there are enough CTAs without a thread per pair (fewer: latency counts, and one thread's chain is shorter there)
+    // Rows of at least a CTA's 256 threads of 8 elements, and enough of them that a thread per pair would take turns: below, latency counts, and one
+    // thread's chain is shorter there.  This kernel against the one below, us (elements a row x tokens): 2,560 x 64 2.5 / 1.9, x 200 2.7 / 2.9, x 512 3.4 / 5.4;
+    // 6,144 x 64 2.9 / 2.9, x 100 2.9 / 3.1, x 200 3.3 / 5.1; 10,240 x 64 3.7 / 3.4, x 100 3.8 / 4.5; 384 x 2,048 4.8 / 3.9.
     auto wide = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (T >= 64 && qkv_is_f16 && !ex && pf0 == nullptr && pf1 == nullptr && D % 8 == 0 && n_rot % 16 == 0 && n_rot > 0 && wide(qkv) && wide(q_out) && wide(kc) && wide(vc)) {
+    const long width = (long)(Hq + 2 * Hkv) * D;
+    if (T >= 64 && width >= 2048 && T * width >= 768 * 1024 && qkv_is_f16 && !ex && pf0 == nullptr && pf1 == nullptr && D % 8 == 0 && n_rot % 16 == 0 && n_rot > 0 && wide(qkv) && wide(q_out) && wide(kc) && wide(vc)) {
         DLP_CHECK_CUDA(launch_pdl(rope_rows_kernel, dim3(T), dim3(256), (size_t)(n_rot / 2) * sizeof(float2), s, (const __half*)qkv, pos, slot, inv_freq, q_out, kc, vc,
                                   Hq, Hkv, D, n_rot, page_size, neox, q_scale));
         return 0;

@@ -996,7 +996,7 @@ def test_gemm_split_k_workspace_fixup(t, T, mode):
 
 def test_rope_rows_of_a_prompt():
     """RoPE of many tokens at once (one block a token) against the one-pair-a-thread kernel: whole and partial rotation, both pairings, negative slots."""
-    T, Hq, Hkv, page = 130, 6, 2, 16
+    T, Hq, Hkv, page = 130, 80, 8, 16             # (fewer heads: the other kernel as well)
     for D, n_rot in ((64, 64), (128, 128), (128, 96), (64, 32)):
         for neox in (False, True):
             g = torch.Generator(DEV).manual_seed(D + n_rot)
