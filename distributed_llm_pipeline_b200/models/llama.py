@@ -91,7 +91,9 @@ class LlamaEngine(EngineCore):
         parts = max(b * ns for b, ns in enumerate(self.attn_splits)) * self.Hq
         self.attn_ws = (torch.zeros(parts * self.D, dtype=f32, device=dev), torch.zeros(parts * 2, dtype=f32, device=dev),
                         torch.zeros(max_seqs * self.Hq, dtype=i32, device=dev)) if max(self.attn_splits) > 1 else None
-        self.scratch = None  # fp16 decode buffer for block-quantised weights on the GEMM path (allocated lazily)
+        # where block-quantised weights are unpacked to for prompts and large batches: the engine's own, since a call's would be held by every graph that
+        # holds the call (None: there is no room, or nothing to unpack)
+        self.scratch = self._prompt_scratch() if dev.type == "cuda" and self.max_tokens > 192 and not ops.TWO_PASS_DEQUANT else None
         # decode attention in one launch (RoPE + KV write + split-KV + join of the splits); plain-llama layers with full-width RoPE
         self.attn_onepass = (dev.type == "cuda" and os.environ.get("DLP_ATTN_ONEPASS", "1") == "1" and cfg.rope_dim == self.D
                              and not cfg.qkv_bias and not cfg.qk_norm)
@@ -163,9 +165,19 @@ class LlamaEngine(EngineCore):
                 cache[pages] = flat.view(len(pages), ps, self.Hkv, self.D).permute(0, 2, 1, 3)
         self.truncate_seq(sid, n_keep + tail)
 
-    def _scratch_for(self, *ws):
-        if not ops.TWO_PASS_DEQUANT:   # block-quant decode is fused into the GEMM: no scratch
+    def _prompt_scratch(self):
+        need = [ops.piece_bytes(w, up) for lw in self.w.layers.values() for w, up in ((lw.wqkv, None), (lw.wv, None), (lw.wo, None), (lw.w_gate, lw.w_up), (lw.w_up, None), (lw.w_down, None))
+                if w is not None and w.dense is None and w.wtype.name.startswith("Q")]
+        if self.last_stage and self.w.lm_head is not None and self.w.lm_head.dense is None and self.w.lm_head.wtype.name.startswith("Q"):
+            need.append(ops.piece_bytes(self.w.lm_head))
+        try:
+            return torch.empty(max(need), dtype=torch.uint8, device=self.device) if need else None
+        except torch.OutOfMemoryError:
             return None
+
+    def _scratch_for(self, *ws):
+        if not ops.TWO_PASS_DEQUANT:
+            return self.scratch
         need = 0
         for w in ws:
             if w is not None and w.dense is None and w.wtype.name.startswith("Q"):
@@ -409,8 +421,8 @@ class LlamaEngine(EngineCore):
             tgt.zero_()
         ops.moe_combine(b["y"][:A], b["plan"], b["w"][:A], T, k, tgt)
         if lw.w_gate is not None:        # always-on shared expert, gated (qwen2moe) or not (deepseek, bailingmoe): device ops, no sync
-            act = ops.linear(lw.w_gate, xn, "swiglu", w_up=lw.w_up)
-            ys = ops.linear(lw.w_down, act, "f32")
+            act = ops.linear(lw.w_gate, xn, "swiglu", w_up=lw.w_up, scratch=self._scratch_for(lw.w_gate, lw.w_up))
+            ys = ops.linear(lw.w_down, act, "f32", scratch=self._scratch_for(lw.w_down))
             if lw.shared_gate is not None:
                 tgt.addcmul_(torch.sigmoid(xn.float() @ lw.shared_gate)[:, None], ys)
             else:
@@ -524,7 +536,7 @@ class LlamaEngine(EngineCore):
         """Bytes held on this rank's device by category (`llama_memory_breakdown_print`, llama.h:1501)."""
         def nb(*ts):
             return sum(t.numel() * t.element_size() for t in ts if t is not None)
-        act = nb(self.h, self.delta, self.xn, self.qkv32, self.qkv16, self.q, self.att, self.act, self.logits, *(self.attn_ws or ()))
+        act = nb(self.h, self.delta, self.xn, self.qkv32, self.qkv16, self.q, self.att, self.act, self.logits, *(self.attn_ws or ()), self.scratch)
         return {"model": self.w.nbytes(), "kv_cache": self.kv.bytes(), "compute": act,
                 "graphs": len(self._graphs), "device": str(self.device)}
 

@@ -171,8 +171,11 @@ def linear(w: DeviceWeight, x: torch.Tensor, out_mode: str = "f16", w_up: Device
         if scratch is None or scratch.numel() * scratch.element_size() < need:
             scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
         _count(2 if w_up is not None else 1)
-    elif quant and T > 192 and scratch is None:    # room for a piece of the weights in fp16 (from the caching allocator: safe on any stream)
-        scratch = torch.empty(max(min(PIECE_BYTES, w.N * w.K * (4 if w_up is not None else 2)), w.K * 1024), dtype=torch.uint8, device=x.device)
+    elif quant and T > 192 and scratch is None:    # (from the caching allocator: safe on any stream)
+        try:
+            scratch = torch.empty(piece_bytes(w, w_up), dtype=torch.uint8, device=x.device)
+        except torch.OutOfMemoryError:             # without it the weights are unpacked inside the GEMM, once per 256 tokens
+            pass
     sb = 0 if scratch is None else scratch.numel() * scratch.element_size()
     ws = gemm_workspace(x.device)                 # split-K workspace (skinny problems use every SM)
     L.dlp_linear_ws.restype = C.c_int
@@ -187,6 +190,13 @@ def linear(w: DeviceWeight, x: torch.Tensor, out_mode: str = "f16", w_up: Device
 # fp16 weights unpacked at a time for a prompt.  Llama-8B gate and up in Q4_K, 256 / 1,021 tokens: 218 / 268 us with 32 MB (small GEMMs), 167 / 242
 # with 64, 143 / 244 with 128, 123 / 244 with all 235
 PIECE_BYTES = 128 << 20
+
+
+def piece_bytes(w: DeviceWeight, w_up: DeviceWeight | None = None) -> int:
+    """Scratch with which `linear` unpacks a block-quantised weight for more than 192 tokens in pieces."""
+    return max(min(PIECE_BYTES, w.N * w.K * (4 if w_up is not None else 2)), w.K * 1024)
+
+
 _GEMM_WS: dict = {}
 GEMM_WS_BYTES = int(_os.environ.get("DLP_GEMM_WS_MB", "64")) << 20
 

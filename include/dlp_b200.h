@@ -66,8 +66,11 @@ int dlp_gemm_f16(const void* w0, const void* w1, int ldw, const void* x, int ldx
                  int K, int epilogue, int is_bf16, int split_k, void* stream);
 
 /* Any-T linear layer on any supported weight type.  T<=4 (T in {1,2,4}) routes to dlp_gemv.  Larger T runs the tcgen05
- * GEMM with the block-quant decode fused into its operand producer; x must be fp16 when T>4.  `scratch` is only used with
- * DLP_GEMM_DEQUANT_SCRATCH=1 (A/B aid: weights are first decoded to fp16 there, 2*N*K bytes per matrix, two for SwiGLU).
+ * GEMM with the block-quant decode fused into its operand producer; x must be fp16 when T>4.  `scratch` (NULL: none) is written for block types
+ * with T>192, K a multiple of 256, when it is 16-byte aligned and holds at least 256 rows of fp16 (512*K bytes, 1024*K for SwiGLU): the weights are
+ * unpacked there in pieces, which is faster than decoding them once per 256 tokens; without it, or with less, they are decoded in the GEMM.
+ * Calls that share one scratch must not overlap on the GPU.  With DLP_GEMM_DEQUANT_SCRATCH=1 (A/B aid) every T>4 decodes whole matrices there,
+ * 2*N*K bytes each, two for SwiGLU, and a smaller scratch is an error.
  * ref: ggml_cuda_mul_mat dispatch (ggml-cuda/ggml-cuda.cu:2182-2265) incl. dequantise-then-cuBLAS (:1287-1294). */
 int dlp_linear(const dlp_weight* w0, const dlp_weight* w1, const void* x, const float* norm_w, float eps, void* y,
                int ldy, int out_mode, int T, void* scratch, size_t scratch_bytes, void* stream);

@@ -221,3 +221,17 @@ def test_decode_attention_changes_its_form_with_the_context(tmp_models):
         assert ("cluster" in forms and True in forms) == cluster
         logits.append(torch.stack(rows))
     assert nmse(*logits) < 1e-6
+
+
+def test_prompt_scratch_belongs_to_the_engine(tmp_models):
+    """Where block types are unpacked to is allocated once, counted, and not held again by a graph whose batch is large enough to use it."""
+    eng = LlamaEngine(load_weights(tmp_models[("tiny", "Q8_0")], "cuda"), n_ctx=64, max_seqs=200, page_size=16, max_batch_tokens=256)
+    assert eng.scratch is not None and eng.memory_breakdown()["compute"] > eng.scratch.numel()
+    before, sids = eng.scratch.data_ptr(), [eng.alloc_seq() for _ in range(200)]
+    want = eng.decode(sids, [3 + i % 50 for i in range(200)], sample=False, use_graph=False).clone()
+    for sid in sids:
+        eng.truncate_seq(sid, 0)
+    got = eng.decode(sids, [3 + i % 50 for i in range(200)], sample=False)
+    assert nmse(want, got) < 1e-9 and eng.scratch.data_ptr() == before
+    few = LlamaEngine(load_weights(tmp_models[("tiny", "Q8_0")], "cuda"), n_ctx=64, max_seqs=1, page_size=16, max_batch_tokens=64)
+    assert few.scratch is None

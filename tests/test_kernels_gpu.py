@@ -288,6 +288,21 @@ def test_linear_quant_two_pass_scratch_entry_point():
     assert rc == 0 and nmse(x.float() @ exact.T, y) < 5e-6
 
 
+def test_prompt_without_room_for_pieces(monkeypatch):
+    """More than 192 tokens on block types where nothing can be allocated: the weights are unpacked in the GEMM instead."""
+    w, exact = _w(512, 1024, GGMLType.Q4_K, 1)
+    x = torch.randn(300, 1024, device=DEV, generator=torch.Generator(DEV).manual_seed(3)).half()
+    out, empty = torch.empty(300, 512, device=DEV), torch.empty
+
+    def full(*a, dtype=None, **kw):
+        if dtype == torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*a, dtype=dtype, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    ops.linear(w, x, "f32", out=out)
+    assert nmse(x.double() @ exact.double().T, out) < 2e-7
+
+
 def test_products_with_an_operand_unpacked_just_before():
     """Rows unpacked by one launch are the weights of the next, which may be requested early only where nothing writes them: different weights through
     one buffer, back to back, against 64 bits (fp16 values, fp32 sums)."""
