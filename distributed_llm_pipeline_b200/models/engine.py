@@ -131,6 +131,12 @@ class NullComm:
     fused = False
 
 
+def host_copy(t: torch.Tensor) -> torch.Tensor:
+    """`t` for a copy to the device that does not wait: a pinned tensor would be read when the stream gets there, with what its owner has put into it by then; from
+    pageable memory the values are taken before the copy returns."""
+    return t.clone() if t.device.type == "cpu" and t.is_pinned() else t
+
+
 class EngineCore:
     def _init_core(self, weights, n_ctx: int, max_seqs: int, page_size: int, max_batch_tokens: int, comm, first_stage: bool, last_stage: bool, device):
         """Everything that does not depend on the model family; the caller allocates `kv`, `rstate` and the activation buffers."""
@@ -302,7 +308,7 @@ class EngineCore:
             self.active[:B].copy_(torch.tensor(sids, dtype=torch.int32), non_blocking=False)
             self._active_host = list(sids)
         if tokens is not None and self.first_stage:
-            self.next_tok[:B].copy_(torch.as_tensor(tokens, dtype=torch.int32), non_blocking=True)
+            self.next_tok[:B].copy_(host_copy(torch.as_tensor(tokens, dtype=torch.int32)), non_blocking=True)
         if hidden_in is not None:
             self.h[:B].copy_(hidden_in)
         graphable = (use_graph and self.eval_callback is None and self.device.type == "cuda" and self._graph_ok()

@@ -526,7 +526,7 @@ class LayeredEngine(EngineCore):
         """Pooled final-norm hidden states of `tokens` (`mean` | `last` | `cls` | `none`), in a scratch sequence slot."""
         if pooling not in ("mean", "last", "cls", "none"):
             raise ValueError(f"unknown pooling {pooling!r}")
-        tokens = list(tokens)
+        tokens = tokens.tolist() if isinstance(tokens, torch.Tensor) else list(tokens)
         if len(tokens) > self.max_tokens:
             raise ValueError(f"{len(tokens)} tokens exceed the batch limit {self.max_tokens}")
         sid = self.alloc_seq()

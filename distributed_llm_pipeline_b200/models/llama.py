@@ -18,7 +18,7 @@ import torch
 
 from ..ops import api as ops
 from ..ops import lib as _lib
-from .engine import EngineCore, NullComm, PagedKVCache, Sequence  # noqa: F401 (Sequence, NullComm: part of this module's surface)
+from .engine import EngineCore, NullComm, PagedKVCache, Sequence, host_copy  # noqa: F401 (Sequence, NullComm: part of this module's surface)
 from .reference import limit_to_groups, rope_attn_scale, rope_inv_freq
 from .weights import ModelWeights
 
@@ -651,7 +651,7 @@ class LlamaEngine(EngineCore):
             self.slot[:T].copy_(slot.to(torch.int32), non_blocking=True)
             sp = self.sp_ok and T > 4
             if self.first_stage:
-                self.tokens[:T].copy_(tokens[c0:c0 + T], non_blocking=True)
+                self.tokens[:T].copy_(host_copy(tokens[c0:c0 + T]), non_blocking=True)
                 if not sp:
                     self._embed(T)
             else:

@@ -235,3 +235,23 @@ def test_prompt_scratch_belongs_to_the_engine(tmp_models):
     assert nmse(want, got) < 1e-9 and eng.scratch.data_ptr() == before
     few = LlamaEngine(load_weights(tmp_models[("tiny", "Q8_0")], "cuda"), n_ctx=64, max_seqs=1, page_size=16, max_batch_tokens=64)
     assert few.scratch is None
+
+
+def test_tokens_in_pinned_memory_are_taken_at_the_call(tmp_models):
+    """A pinned buffer of token ids may be filled again as soon as the call has returned, although nothing waits for the stream."""
+    eng = LlamaEngine(load_weights(tmp_models[("tiny", "F16")], "cuda"), n_ctx=256, max_seqs=1, page_size=16, max_batch_tokens=64)
+    ids = torch.arange(3, 43, dtype=torch.int32)
+    sid = eng.alloc_seq()
+    want = [eng.prefill(sid, ids).clone(), eng.decode([sid], torch.tensor([7]), sample=False).clone()]
+    eng.truncate_seq(sid, 0)
+    buf, one = ids.pin_memory(), torch.tensor([7], dtype=torch.int32).pin_memory()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)                  # the stream is busy for some 10 ms
+    got = eng.prefill(sid, buf)
+    buf.fill_(5)
+    got = [got.clone()]
+    torch.cuda._sleep(20_000_000)
+    lg = eng.decode([sid], one, sample=False)
+    one.fill_(9)
+    got.append(lg.clone())
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
