@@ -68,8 +68,8 @@ __device__ __forceinline__ void split_h2(float a, float b, uint32_t& hi, uint32_
 // sum that is kept: each takes 16 products from zero, parts apart, and the sums over them are rounded fp32 additions.  Error against 64 bits
 // before the output's rounding, 32 heads over 8, D = 128, keys of deviation 1.5: 700 keys 2.4e-7 (fp32 FMA per key 2.4e-7, sums kept in the MMAs
 // 4.1e-7), 32,000 3.1e-7 (3.4e-7, 8.3e-7).
-// 32,000 keys of 8 KV heads of 4 query heads, D = 128 (131 MB): 28.5 us (4.6 TB/s; 108 us with fp32 FMA per key in 128 CTAs); 32 queries
-// of up to 2,000 keys (135 MB): 34 us (117 us).
+// 32,000 keys of 8 KV heads of 4 query heads, D = 128 (131 MB): 28.7 us (4.6 TB/s; 108 us with fp32 FMA per key in 128 CTAs); 32 queries
+// of 2,000 keys each (262 MB): 42 us (172 us).
 //   ROPE: takes the fp32 row of the QKV mat-vec, rotates q in registers, writes the new token's K and V and uses them from shared memory.
 constexpr int ATTN_KEYS_MIN = 128;      // keys a split is worth: 2 tiles per warp, all requested before the dependency wait (700 keys in a
                                         // decode step: as fast as the cluster form; with 256 keys 1.7 us slower)

@@ -98,8 +98,9 @@ int gemm_quant(const QWeight& w0, const QWeight* w1, int wtype, const void* x, i
     int bt = grp ? grp->bt : (T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256);
     const QWeight up = w1 ? *w1 : QWeight();
     // Token tiles of up to 64 stream the weights' bytes (gemm_quant_small.cuh); wider ones are bound by the MMAs.  At 64 tokens the
-    // bytes still bound it (Q8_0 gate and up of Llama-8B: 35 us, 7 tokens 34), up to 192 some tiles of 64 are faster than
-    // unpacking the weights for one pass (Q4_K gate and up, 192 tokens: 120 us against 137; 256 tokens: 160 against 143).
+    // bytes still bound it (Q8_0 gate and up of Llama-8B: 35 us, 7 tokens 34), up to 192 some tiles of 64 are mostly faster than unpacking the
+    // weights for one pass.  192 tokens in tiles / 193 in one pass, us: gate and up of 14336 x 4096 in Q8_0 88 / 143, Q4_K 119 / 138, Q5_K 132 / 140, Q6_K
+    // 132 / 130; 4096 x 14336 38 / 63, 45 / 61, 50 / 62, 84 / 57; 2048 x 2048 6.9 / 12.1, 8.6 / 11.7, 9.2 / 11.8, 8.4 / 11.4.  Four tiles of 64 in Q4_K: 160 / 143.
     if ((bt <= 64 || (grp == nullptr && T <= 192)) && coll == nullptr && epilogue != EPI_RS_PUSH_F32 && gemm_quant_small_takes(w0, wtype) && (na == 1 || gemm_quant_small_takes(up, wtype))) {
         if (bt > 64) bt = 64;
         CUtensorMap tx;

@@ -409,7 +409,9 @@ class LlamaEngine(EngineCore):
         ops.linear(lw.router_wp, xn, "f32", out=b["logits"][:T])     # router (padded to a full 128-row tile for the GEMM sizes)
         ops.moe_route_ex(b["logits"][:T], nE, k, cfg.moe_norm_topk, b["ids"][:A], b["w"][:A])
         per = max(1, A // nE)
-        bt = 16 if per <= 16 else 32 if per <= 32 else 64 if per <= 96 or lw.e_gate_s.wtype.name.startswith("Q") else 128      # (block types: gemm_quant_small.cuh)
+        # block types at every length in tiles of 64 (gemm_quant_small.cuh): two layers of Mixtral in Q4_K_M, 1,000 / 3,000 tokens 3.8 / 10.6 ms, in tiles of 128 (the
+        # weights unpacked in the GEMM of gemm_tcgen05.cuh) 8.0 / 23.0; in Q8_0 3.2 / 9.7 against 6.3 / 18.0
+        bt = 16 if per <= 16 else 32 if per <= 32 else 64 if per <= 96 or lw.e_gate_s.wtype.name.startswith("Q") else 128
         ops.moe_plan(b["ids"][:A], nE, bt, b["plan"])
         ops.moe_gather(xn, b["plan"], k, A, b["xs"][:A])
         ops.linear_grouped(lw.e_gate_s, b["xs"][:A], b["act"][:A], "swiglu", nE, F, bt, b["plan"], w_up=lw.e_up_s)

@@ -232,7 +232,7 @@ def test_prompt_scratch_belongs_to_the_engine(tmp_models):
     for sid in sids:
         eng.truncate_seq(sid, 0)
     got = eng.decode(sids, [3 + i % 50 for i in range(200)], sample=False)
-    assert nmse(want, got) < 1e-9 and eng.scratch.data_ptr() == before
+    assert nmse(want, got) < 1e-6 and eng.scratch.data_ptr() == before      # (small tiles add their splits with atomics)
     few = LlamaEngine(load_weights(tmp_models[("tiny", "Q8_0")], "cuda"), n_ctx=64, max_seqs=1, page_size=16, max_batch_tokens=64)
     assert few.scratch is None
 

@@ -1061,3 +1061,31 @@ def test_a_wait_that_runs_out_is_an_error_once(tmp_models):
     finally:
         L.check(lib.dlp_set_wait_limit(2.0), "set_wait_limit")
     assert lib.dlp_set_wait_limit(0.0) != 0
+
+
+@pytest.mark.parametrize("t,bt", [(GGMLType.F16, 64), (GGMLType.F16, 128), (GGMLType.BF16, 128), (GGMLType.Q4_K, 64), (GGMLType.Q8_0, 64), (GGMLType.Q6_K, 64), (GGMLType.Q5_K, 64)])
+@pytest.mark.parametrize("rows", [[700, 1, 0, 129], [64, 63, 65, 300]])
+def test_grouped_products_of_long_prompts(t, bt, rows):
+    """Experts with several tiles of tokens (dense weights on pairs of SMs, block types in tiles of 64), with one token and with none, against 64 bits."""
+    nE, E, F, A = len(rows), 512, 512 if t.name.startswith("Q") else 384, sum(rows)
+    half = torch.bfloat16 if t == GGMLType.BF16 else torch.float16
+    ids = torch.repeat_interleave(torch.arange(nE), torch.tensor(rows)).to(torch.int32).to(DEV)
+    plan = ops.MoePlan(A, nE, DEV)
+    ops.moe_plan(ids, nE, bt, plan)
+    assert int(plan.n_tiles) == sum((n + bt - 1) // bt for n in rows)
+    (Wg, dg), (Wu, du), (Wd, dd) = _w(nE * F, E, t, 1), _w(nE * F, E, t, 2), _w(nE * E, F, t, 3)
+    x = torch.randn(A, E, device=DEV, generator=torch.Generator(DEV).manual_seed(5)).to(half)
+    z = torch.randn(A, F, device=DEV, generator=torch.Generator(DEV).manual_seed(6)).to(half)
+    act, y = torch.zeros(A, F, dtype=torch.float16, device=DEV), torch.zeros(A, E, device=DEV)
+    if t != GGMLType.BF16:            # (the gated epilogue of bf16 weights is bf16)
+        ops.linear_grouped(Wg, x, act, "swiglu", nE, F, bt, plan, w_up=Wu)
+    ops.linear_grouped(Wd, z, y, "f32", nE, E, bt, plan)
+    at = 0
+    for e, n in enumerate(rows):
+        if n:
+            xe, ze = x[at:at + n].double(), z[at:at + n].double()
+            g, u, d = (m[e * r:(e + 1) * r].double() for m, r in ((dg, F), (du, F), (dd, E)))
+            assert nmse(ze @ d.T, y[at:at + n]) < 2e-7, e
+            if t != GGMLType.BF16:
+                assert nmse(torch.nn.functional.silu(xe @ g.T) * (xe @ u.T), act[at:at + n]) < 2e-6, e
+        at += n
