@@ -10,7 +10,7 @@
 // and epilogue hide behind the other's stream.
 // Llama-8B shapes in us, 7 tokens: Q8_0 gate and up 123 -> 34 (floor of the bytes 19), 4096 x 14336 53 -> 16.5 (9.6), 128256 x 4096 109 (86);
 // Q4_K gate and up 38 (10), 4096 x 14336 20 (5), 128256 x 4096 120 (45): unpacking bounds the 4- and 6-bit types (some 5 instructions a weight
-// with one group of unpacking warps and unpacked FMAs: 150).  Mixtral gate and up of 8 experts in Q4_K, 16 tokens: 1,104 -> 230.
+// with one group of unpacking warps and unpacked FMAs: 150).  Mixtral gate and up of 8 experts in Q4_K, 16 tokens: 1,104 -> 189.
 #pragma once
 #include "gemm_tcgen05.cuh"
 

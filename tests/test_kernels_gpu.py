@@ -1067,7 +1067,7 @@ def test_a_wait_that_runs_out_is_an_error_once(tmp_models):
 @pytest.mark.parametrize("rows", [[700, 1, 0, 129], [64, 63, 65, 300]])
 def test_grouped_products_of_long_prompts(t, bt, rows):
     """Experts with several tiles of tokens (dense weights on pairs of SMs, block types in tiles of 64), with one token and with none, against 64 bits."""
-    nE, E, F, A = len(rows), 512, 512 if t.name.startswith("Q") else 384, sum(rows)
+    nE, E, F, A = len(rows), 768, 512, sum(rows)
     half = torch.bfloat16 if t == GGMLType.BF16 else torch.float16
     ids = torch.repeat_interleave(torch.arange(nE), torch.tensor(rows)).to(torch.int32).to(DEV)
     plan = ops.MoePlan(A, nE, DEV)
